@@ -222,12 +222,12 @@ static splat_status_t scene_pack(splat_scene* s, cudaStream_t st) {
                                      s->d_bvh_pos, st);
     if (e != cudaSuccess) return cuda_fail(e, "pack hit records");
     if (s->d_nodes && s->d_links) {
-        e = launch_refit_tree(s->d_nodes, false, s->n_nodes, s->d_links, s->d_flags, s->d_bvh, s->d_ftri, s->d_scale,
+        e = launch_refit_tree(s->d_nodes, false, s->d_nodes4, s->n_nodes, s->d_links, s->d_flags, s->d_bvh, s->d_ftri, s->d_scale,
                               s->pad_rel, st);
         if (e != cudaSuccess) return cuda_fail(e, "BVH refit");
     }
     if (s->d_nodes4 && s->d_links4) {
-        e = launch_refit_tree(s->d_nodes4, true, s->n_nodes4, s->d_links4, s->d_flags, s->d_bvh, s->d_ftri, s->d_scale,
+        e = launch_refit_tree(s->d_nodes4, true, s->d_nodes4, s->n_nodes4, s->d_links4, s->d_flags, s->d_bvh, s->d_ftri, s->d_scale,
                               s->pad_rel, st);
         if (e != cudaSuccess) return cuda_fail(e, "BVH4 refit");
     }
@@ -527,7 +527,7 @@ static splat_status_t hit_any(const splat_scene_t* s, int32_t hitter, const RayS
             e = launch_hit_bvh4(src, cap, Bvh4View{s->d_nodes4, s->d_bvh}, hit_idx, hit_t, s->d_err,
                                 sm_count_current(), st);
         } else {
-            e = launch_hit_bvh(src, cap, BvhView{s->d_nodes, s->d_bvh}, hit_idx, hit_t, s->d_err, sm_count_current(),
+            e = launch_hit_bvh(src, cap, BvhView{s->d_nodes, s->d_bvh, s->d_nodes4}, hit_idx, hit_t, s->d_err, sm_count_current(),
                                st);
         }
     } else if (hitter == SPLAT_HITTER_BRUTE) {

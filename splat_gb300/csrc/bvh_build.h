@@ -23,6 +23,7 @@ struct BvhHost {
 };
 
 bool build_bvh(const splat_ftri_t* tris, int64_t n_tris, BvhHost& out, std::string& err);
-void prim_box(const splat_ftri_t& t, float pad_abs, float pad_rel, float lo[3], float hi[3]);
+// Padded box of a triangle in a frame.
+void prim_box(const splat_ftri_t& t, const BvhFrame& f, float pad_abs, float pad_rel, float lo[3], float hi[3]);
 
 }  // namespace splat

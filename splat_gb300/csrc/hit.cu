@@ -498,8 +498,8 @@ __global__ void __launch_bounds__(kBvhThreads) hit_bvh_kernel(RaySrc src, BvhVie
     for_each_ray(n, src.fetch, [&](int64_t kk) {
         const int64_t k = src.perm ? (int64_t)src.perm[kk] : kk;
         const HitRay r = load_hit_ray<AOS>(src, k);
-        const float ix = safe_inv(r.dx), iy = safe_inv(r.dy), iz = safe_inv(r.dz);
-        const float oix = r.ox * ix, oiy = r.oy * iy, oiz = r.oz * iz;
+        const SlabRay sr = slab_ray(r, bvh.root4);
+        const float ix = sr.ix, iy = sr.iy, iz = sr.iz, oix = sr.oix, oiy = sr.oiy, oiz = sr.oiz;
         float best = __int_as_float(0x7f800000);
         int32_t bi = 1;
         int sp = 0;
@@ -861,13 +861,16 @@ cudaError_t launch_pack_hits(const splat_ftri_t* ftri, int64_t n_tris, TriHit* b
     return cudaGetLastError();
 }
 
-__device__ __forceinline__ void leaf_box(int ref, const TriHit* recs, const splat_ftri_t* ftri, float pad_abs,
-                                         float pad_rel, float lo[3], float hi[3]) {
+__device__ __forceinline__ void leaf_box(int ref, const TriHit* recs, const splat_ftri_t* ftri, const BvhFrame& fr,
+                                         float pad_abs, float pad_rel, float lo[3], float hi[3]) {
     const int enc = ~ref;
     const int first = enc >> 4, count = (enc & 15) + 1;
     for (int j = 0; j < count; ++j) {
         const int32_t idx = __float_as_int(recs[first + j].a_idx.w);
-        const float* p = ftri[idx - 1].v[1];
+        const float* q = ftri[idx - 1].v[1];
+        float p[9];
+        for (int v = 0; v < 9; ++v) p[v] = q[v];
+        for (int v = 0; v < 3; ++v) to_frame(fr, p[3 * v], p[3 * v + 1], p[3 * v + 2]);
         float tl[3], th[3];
         for (int a = 0; a < 3; ++a) {
             tl[a] = fminf(fminf(p[a], p[3 + a]), p[6 + a]);
@@ -891,7 +894,7 @@ __device__ __forceinline__ void leaf_box(int ref, const TriHit* recs, const spla
 __device__ __forceinline__ float4 ldcg4(const float4* p) { return __ldcg(p); }
 
 __device__ __forceinline__ void refit2_node(BvhNode* nodes, int q, const TriHit* recs, const splat_ftri_t* ftri,
-                                            float pad_abs, float pad_rel) {
+                                            const BvhFrame& fr, float pad_abs, float pad_rel) {
     const int4 c = nodes[q].c;
     float l[2][3], h[2][3];
     const int refs[2] = {c.x, c.y};
@@ -909,7 +912,7 @@ __device__ __forceinline__ void refit2_node(BvhNode* nodes, int q, const TriHit*
             l[i][2] = fminf(z.x, z.z);
             h[i][2] = fmaxf(z.y, z.w);
         } else {
-            leaf_box(refs[i], recs, ftri, pad_abs, pad_rel, l[i], h[i]);
+            leaf_box(refs[i], recs, ftri, fr, pad_abs, pad_rel, l[i], h[i]);
         }
     }
     nodes[q].x = make_float4(l[0][0], h[0][0], l[1][0], h[1][0]);
@@ -918,7 +921,7 @@ __device__ __forceinline__ void refit2_node(BvhNode* nodes, int q, const TriHit*
 }
 
 __device__ __forceinline__ void refit4_node(Bvh4Node* nodes, int q, const TriHit* recs, const splat_ftri_t* ftri,
-                                            float pad_abs, float pad_rel) {
+                                            const BvhFrame& fr, float pad_abs, float pad_rel) {
     const int nc = nodes[q].meta.x;
     const int4 c = nodes[q].c;
     const int refs[4] = {c.x, c.y, c.z, c.w};
@@ -941,7 +944,7 @@ __device__ __forceinline__ void refit4_node(Bvh4Node* nodes, int q, const TriHit
                     h[2] = fmaxf(h[2], comp(hz, j));
                 }
             } else {
-                leaf_box(refs[i], recs, ftri, pad_abs, pad_rel, l, h);
+                leaf_box(refs[i], recs, ftri, fr, pad_abs, pad_rel, l, h);
             }
         }
         for (int a = 0; a < 3; ++a) {
@@ -959,17 +962,19 @@ __device__ __forceinline__ void refit4_node(Bvh4Node* nodes, int q, const TriHit
 }
 
 template <bool WIDE>
-__global__ void refit_tree_kernel(void* nodes_v, int64_t n_nodes, const int32_t* __restrict__ links, unsigned* flags,
+__global__ void refit_tree_kernel(void* nodes_v, const Bvh4Node* root4, int64_t n_nodes,
+                                  const int32_t* __restrict__ links, unsigned* flags,
                                   const TriHit* __restrict__ recs, const splat_ftri_t* __restrict__ ftri,
                                   const unsigned* __restrict__ scale, float pad_rel) {
     const float pad_abs = pad_abs_of_scale(__uint_as_float(*scale));
+    const BvhFrame fr = root_frame(root4);  // a refit writes no meta
     for (int64_t q0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q0 < n_nodes;
          q0 += (int64_t)gridDim.x * blockDim.x) {
         if (links[n_nodes + q0] != 0) continue;  // has inner children: reached by its last child
         int q = (int)q0;
         for (int64_t guard = 0; guard < n_nodes; ++guard) {
-            if (WIDE) refit4_node(reinterpret_cast<Bvh4Node*>(nodes_v), q, recs, ftri, pad_abs, pad_rel);
-            else refit2_node(reinterpret_cast<BvhNode*>(nodes_v), q, recs, ftri, pad_abs, pad_rel);
+            if (WIDE) refit4_node(reinterpret_cast<Bvh4Node*>(nodes_v), q, recs, ftri, fr, pad_abs, pad_rel);
+            else refit2_node(reinterpret_cast<BvhNode*>(nodes_v), q, recs, ftri, fr, pad_abs, pad_rel);
             const int p = links[q];
             if (p < 0) break;
             __threadfence();
@@ -980,18 +985,18 @@ __global__ void refit_tree_kernel(void* nodes_v, int64_t n_nodes, const int32_t*
     }
 }
 
-cudaError_t launch_refit_tree(void* nodes, bool wide, int64_t n_nodes, const int32_t* links, unsigned* flags,
-                              const TriHit* bvh_recs, const splat_ftri_t* ftri, const unsigned* scale, float pad_rel,
-                              cudaStream_t s) {
+cudaError_t launch_refit_tree(void* nodes, bool wide, const Bvh4Node* root4, int64_t n_nodes, const int32_t* links,
+                              unsigned* flags, const TriHit* bvh_recs, const splat_ftri_t* ftri,
+                              const unsigned* scale, float pad_rel, cudaStream_t s) {
     if (n_nodes <= 0) return cudaSuccess;
     cudaError_t e = cudaMemsetAsync(flags, 0, sizeof(unsigned) * (size_t)n_nodes, s);
     if (e != cudaSuccess) return e;
     if (wide)
-        refit_tree_kernel<true><<<grid_for(n_nodes, 128, 152, 8), 128, 0, s>>>(nodes, n_nodes, links, flags, bvh_recs,
-                                                                             ftri, scale, pad_rel);
+        refit_tree_kernel<true><<<grid_for(n_nodes, 128, 152, 8), 128, 0, s>>>(nodes, root4, n_nodes, links, flags,
+                                                                             bvh_recs, ftri, scale, pad_rel);
     else
-        refit_tree_kernel<false><<<grid_for(n_nodes, 128, 152, 8), 128, 0, s>>>(nodes, n_nodes, links, flags, bvh_recs,
-                                                                              ftri, scale, pad_rel);
+        refit_tree_kernel<false><<<grid_for(n_nodes, 128, 152, 8), 128, 0, s>>>(nodes, root4, n_nodes, links, flags,
+                                                                              bvh_recs, ftri, scale, pad_rel);
     ++g_launches;
     return cudaGetLastError();
 }

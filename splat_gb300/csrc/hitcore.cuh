@@ -101,6 +101,26 @@ __device__ __forceinline__ float safe_inv(float d) {
     return 1.0f / (fabsf(d) > 1.0e-30f ? d : copysignf(1.0e-30f, d));
 }
 
+// The slab-test terms of a ray in the tree's frame: inverse direction and
+// origin times inverse direction.
+struct SlabRay {
+    float ix, iy, iz, oix, oiy, oiz;
+};
+__device__ __forceinline__ SlabRay slab_ray(const HitRay& r, const Bvh4Node* root) {
+    const BvhFrame f = root_frame(root);
+    float ox = r.ox, oy = r.oy, oz = r.oz, dx = r.dx, dy = r.dy, dz = r.dz;
+    to_frame(f, ox, oy, oz);
+    to_frame(f, dx, dy, dz);
+    SlabRay s;
+    s.ix = safe_inv(dx);
+    s.iy = safe_inv(dy);
+    s.iz = safe_inv(dz);
+    s.oix = ox * s.ix;
+    s.oiy = oy * s.iy;
+    s.oiz = oz * s.iz;
+    return s;
+}
+
 __device__ __forceinline__ float comp(const float4& v, int i) {
     return i == 0 ? v.x : (i == 1 ? v.y : (i == 2 ? v.z : v.w));
 }
@@ -164,8 +184,7 @@ __device__ __forceinline__ void bvh4_closest(const HitRay& r, const Bvh4View& bv
                                              float& best_out, int32_t& bi_out, WorkCount* wc = nullptr) {
     const float kInf = __int_as_float(0x7f800000);
     const float kMax = 3.402823466e38f;
-    const float ix = safe_inv(r.dx), iy = safe_inv(r.dy), iz = safe_inv(r.dz);
-    const float oix = r.ox * ix, oiy = r.oy * iy, oiz = r.oz * iz;
+    const SlabRay sr = slab_ray(r, bvh.nodes);
     float best = kInf;
     int32_t bi = 1;
     int sp = 0;
@@ -176,7 +195,7 @@ __device__ __forceinline__ void bvh4_closest(const HitRay& r, const Bvh4View& bv
             if (wc) ++wc->nodes;
             const int4 c = __ldg(&nd->c);
             float tmin[4], tmax[4], key[4];
-            node4_slabs(nd, ix, iy, iz, oix, oiy, oiz, tmin, tmax);
+            node4_slabs(nd, sr.ix, sr.iy, sr.iz, sr.oix, sr.oiy, sr.oiz, tmin, tmax);
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
                 const bool h = (tmin[i] <= tmax[i]) & (tmin[i] <= best);  // tmin: clamped at 0; empty slots fail
@@ -257,7 +276,8 @@ __device__ __forceinline__ void bvh4_refill_loop(int64_t n, unsigned long long* 
     int2 stack[kBvhStack];
     HitRay r{};
     Bvh4View bvh{};
-    float ix = 0.f, iy = 0.f, iz = 0.f, oix = 0.f, oiy = 0.f, oiz = 0.f, best = kInf;
+    SlabRay sr{};
+    float best = kInf;
     int32_t bi = 1;
     int sp = 0, node = kDone, visits = 0;
     int64_t k = 0;
@@ -276,12 +296,7 @@ __device__ __forceinline__ void bvh4_refill_loop(int64_t n, unsigned long long* 
                     k = (int64_t)kk;
                     r = load(k);
                     bvh = view(k);
-                    ix = safe_inv(r.dx);
-                    iy = safe_inv(r.dy);
-                    iz = safe_inv(r.dz);
-                    oix = r.ox * ix;
-                    oiy = r.oy * iy;
-                    oiz = r.oz * iz;
+                    sr = slab_ray(r, bvh.nodes);
                     best = kInf;
                     bi = 1;
                     sp = 0;
@@ -299,7 +314,7 @@ __device__ __forceinline__ void bvh4_refill_loop(int64_t n, unsigned long long* 
             const Bvh4Node* nd = bvh.nodes + node;
             const int4 c = __ldg(&nd->c);
             float tmin[4], tmax[4], key[4];
-            node4_slabs(nd, ix, iy, iz, oix, oiy, oiz, tmin, tmax);
+            node4_slabs(nd, sr.ix, sr.iy, sr.iz, sr.oix, sr.oiy, sr.oiz, tmin, tmax);
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
                 const bool h = (tmin[i] <= tmax[i]) & (tmin[i] <= best);  // tmin: clamped at 0; empty slots fail
@@ -379,8 +394,7 @@ __device__ __forceinline__ void bvh4_closest_packet(const HitRay& r, bool valid,
                                                     int32_t* err, float& best_out, int32_t& bi_out,
                                                     WorkCount* wc = nullptr) {
     const float kInf = __int_as_float(0x7f800000);
-    const float ix = safe_inv(r.dx), iy = safe_inv(r.dy), iz = safe_inv(r.dz);
-    const float oix = r.ox * ix, oiy = r.oy * iy, oiz = r.oz * iz;
+    const SlabRay sr = slab_ray(r, bvh.nodes);
     float best = kInf;
     float reach = kInf;  // the largest best hit over the warp's valid lanes
     int32_t bi = 1;
@@ -392,7 +406,7 @@ __device__ __forceinline__ void bvh4_closest_packet(const HitRay& r, bool valid,
             if (wc && valid) ++wc->nodes;
             const int4 c = __ldg(&nd->c);
             float tmin[4], tmax[4];
-            node4_slabs(nd, ix, iy, iz, oix, oiy, oiz, tmin, tmax);
+            node4_slabs(nd, sr.ix, sr.iy, sr.iz, sr.oix, sr.oiy, sr.oiz, tmin, tmax);
             unsigned u[4];
 #pragma unroll
             for (int i = 0; i < 4; ++i) {

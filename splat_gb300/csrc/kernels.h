@@ -65,9 +65,53 @@ static_assert(sizeof(BvhNode) == 64, "BvhNode layout");
 struct __align__(16) Bvh4Node {
     float4 lox, hix, loy, hiy, loz, hiz;
     int4 c;      // child refs (as BvhNode)
-    int4 meta;   // x: number of children (2..4)
+    int4 meta;   // x: number of children (2..4); root: y, z, w the tree's frame (frame_of)
 };
 static_assert(sizeof(Bvh4Node) == 128, "Bvh4Node layout");
+
+// The frame a scene's BVH boxes are axis-aligned in, as rows of a matrix
+// applied to world positions and directions.  A linear map keeps the t of
+// every ray-box intersection, so traversal rotates each ray once (slab_ray)
+// and tests triangles in world space as before; only how tightly the boxes
+// fit changes.  The frame is the vector part of a unit quaternion with
+// w >= 0, kept as float bits in the four-wide root's meta.y, z, w; all zero
+// is the world frame.  Host build, refit and traversal derive the matrix
+// with the same binary32 operations.
+struct BvhFrame {
+    float r[9];
+    bool world;
+};
+__host__ __device__ __forceinline__ BvhFrame frame_of(float x, float y, float z) {
+    BvhFrame f;
+    f.world = x == 0.0f && y == 0.0f && z == 0.0f;
+    const float w2 = 1.0f - ((x * x + y * y) + z * z);
+    const float w = sqrtf(w2 > 0.0f ? w2 : 0.0f);
+    f.r[0] = 1.0f - 2.0f * (y * y + z * z);
+    f.r[1] = 2.0f * (x * y - z * w);
+    f.r[2] = 2.0f * (x * z + y * w);
+    f.r[3] = 2.0f * (x * y + z * w);
+    f.r[4] = 1.0f - 2.0f * (x * x + z * z);
+    f.r[5] = 2.0f * (y * z - x * w);
+    f.r[6] = 2.0f * (x * z - y * w);
+    f.r[7] = 2.0f * (y * z + x * w);
+    f.r[8] = 1.0f - 2.0f * (x * x + y * y);
+    return f;
+}
+__host__ __device__ __forceinline__ void to_frame(const BvhFrame& f, float& x, float& y, float& z) {
+    if (f.world) return;
+    const float a = (f.r[0] * x + f.r[1] * y) + f.r[2] * z;
+    const float b = (f.r[3] * x + f.r[4] * y) + f.r[5] * z;
+    const float c = (f.r[6] * x + f.r[7] * y) + f.r[8] * z;
+    x = a;
+    y = b;
+    z = c;
+}
+#ifdef __CUDACC__
+__device__ __forceinline__ BvhFrame root_frame(const Bvh4Node* root) {
+    const int4 m = __ldg(&root->meta);
+    return frame_of(__int_as_float(m.y), __int_as_float(m.z), __int_as_float(m.w));
+}
+#endif
 
 struct Bvh4View {
     const Bvh4Node* nodes;
@@ -80,6 +124,7 @@ constexpr int kBvhStack = 64;
 struct BvhView {
     const BvhNode* nodes;
     const TriHit* tris;  // BVH order
+    const Bvh4Node* root4;  // the four-wide tree over the same leaves: its root holds the frame
 };
 
 // brute force over prepacked hit records (reference indices 2..T in order),
@@ -105,10 +150,11 @@ cudaError_t read_hit_work(uint64_t out[4], bool reset, cudaStream_t s);
 // grid of a work-counter traversal launch (one resident wave)
 int resident_grid(const void* kernel, int64_t cap, int sm_count, int threads, int max_per_sm);
 // one-launch bottom-up refit of a two-child (wide = false) or four-wide tree;
-// links: parent per node, then number of inner children per node
-cudaError_t launch_refit_tree(void* nodes, bool wide, int64_t n_nodes, const int32_t* links, unsigned* flags,
-                              const TriHit* bvh_recs, const splat_ftri_t* ftri, const unsigned* scale, float pad_rel,
-                              cudaStream_t s);
+// links: parent per node, then number of inner children per node; root4: the
+// four-wide root, whose frame the boxes are taken in
+cudaError_t launch_refit_tree(void* nodes, bool wide, const Bvh4Node* root4, int64_t n_nodes, const int32_t* links,
+                              unsigned* flags, const TriHit* bvh_recs, const splat_ftri_t* ftri,
+                              const unsigned* scale, float pad_rel, cudaStream_t s);
 
 
 // GPU BVH rebuild (lbvh.cu): linear BVH over Morton-sorted centroids, written
