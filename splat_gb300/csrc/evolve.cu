@@ -1,8 +1,7 @@
 // evolve.cu -- evolve_ray over the active rays of one bounce, with the ray
 // compaction (warp ballot + block scan, one atomic per block) fused in.  In
 // trace mode the diffuse rays' final_evolution is fused in as well and the
-// result is compacted into a splat queue; one splat launch per frame then
-// spreads (ray, sample) pairs over full warps.
+// result is compacted into a splat queue for the splat launches.
 //
 // Reference: evolve_ray src/tracer.jl:181-201, partition! src/partition.jl
 // (semantics: the active rays, in any order, and their count),
@@ -10,13 +9,11 @@
 // src/ray_imagers.jl:78-113.  Each ray's Fresnel draw is keyed by its id, so
 // results do not depend on the order compaction leaves the rays in.
 //
-// Splat: one thread per (queued ray, sample); a ray's n_lambda x N x N
-// samples are consecutive, so a warp's lanes share (broadcast-load) one or a
-// few rays.  Fixed-point maps add round(intensity * 2^frac_bits) with warp-aggregated
-// integer atomics (lanes on the same texel are summed by match_any +
-// reduce_add first), which makes the map independent of ray order and
-// bit-exact run to run.  Float maps use plain float atomics, as the
-// reference does.
+// Splat: one lane per queued ray walks the ray's n_lambda x N x N samples.
+// Fixed-point maps add round(intensity * 2^frac_bits) with integer atomics
+// (runs of samples on one texel are summed in a register first), which makes
+// the map independent of ray order and bit-exact run to run.  Float maps use
+// plain float atomics, as the reference does.
 #include "kernels.h"
 #include "optics.cuh"
 
@@ -24,105 +21,6 @@ namespace splat {
 
 constexpr unsigned kFull = 0xffffffffu;
 constexpr int kEvolveThreads = 256;
-
-__device__ __forceinline__ F3 shfl3(F3 v, int src) {
-    return {__shfl_sync(kFull, v.x, src), __shfl_sync(kFull, v.y, src), __shfl_sync(kFull, v.z, src)};
-}
-
-__device__ __forceinline__ RayState shfl_ray(const RayState& r, int src) {
-    RayState q;
-    q.pos = shfl3(r.pos, src);
-    q.dir = shfl3(r.dir, src);
-    q.dpl = shfl3(r.dpl, src);
-    q.dpx = shfl3(r.dpx, src);
-    q.dpy = shfl3(r.dpy, src);
-    q.ddl = shfl3(r.ddl, src);
-    q.ddx = shfl3(r.ddx, src);
-    q.ddy = shfl3(r.ddy, src);
-    q.lam = __shfl_sync(kFull, r.lam, src);
-    q.x = __shfl_sync(kFull, r.x, src);
-    q.y = __shfl_sync(kFull, r.y, src);
-    q.ignore = __shfl_sync(kFull, r.ignore, src);
-    q.medium = __shfl_sync(kFull, r.medium, src);
-    return q;
-}
-
-// Sample s of a ray: s = ix + nd (iy + nd il), the CartesianIndices order of
-// atomic_spectrum_kernel2's threads.
-__device__ __forceinline__ bool sample_of(const SplatParams& sp, const RayState& q, const Tri& T, int s,
-                                          int64_t& off, float& inten) {
-    const int nd = sp.n_delta;
-    const int ix = s % nd;
-    const int iy = (s / nd) % nd;
-    const int il = s / (nd * nd);
-    const float lam = sp.n_lambda > 0 ? sp.spectrum[il] : q.lam;
-    const float xs = q.x + sp.deltas[ix];
-    const float ys = q.y + sp.deltas[iy];
-    int64_t oij;
-    if (!splat_sample(q, T, lam, xs, ys, sp.w, sp.h, oij, inten)) return false;
-    off = oij + (int64_t)il * sp.w * sp.h;
-    return true;
-}
-
-// All 32 lanes call; lanes with ok add their sample.
-__device__ __forceinline__ void accumulate_warp(const SplatParams& sp, bool ok, int64_t off, float inten) {
-    if (sp.accum == SPLAT_ACCUM_I32) {
-        const unsigned act = __ballot_sync(kFull, ok);
-        if (ok) {
-            const int v = __float2int_rn(inten * sp.scale);
-            const unsigned m = __match_any_sync(act, (unsigned long long)off);
-            const int sum = __reduce_add_sync(m, v);
-            if (lane_id() == __ffs(m) - 1) atomicAdd(reinterpret_cast<int*>(sp.map) + off, sum);
-        }
-    } else if (ok) {
-        atomicAdd(reinterpret_cast<float*>(sp.map) + off, inten);
-    }
-}
-
-__device__ __forceinline__ void accumulate_one(const SplatParams& sp, int64_t off, float inten) {
-    if (sp.accum == SPLAT_ACCUM_I32)
-        atomicAdd(reinterpret_cast<int*>(sp.map) + off, __float2int_rn(inten * sp.scale));
-    else
-        atomicAdd(reinterpret_cast<float*>(sp.map) + off, inten);
-}
-
-// Splat the diffuse rays held by the lanes of this warp (all lanes call).
-// Returns the number of samples this lane accumulated.
-__device__ __forceinline__ int splat_warp(const SplatParams& sp, const splat_ftri_t* tris, bool dif,
-                                          const RayState& fe, int32_t ti) {
-    const int S = (sp.n_lambda > 0 ? sp.n_lambda : 1) * sp.n_delta * sp.n_delta;
-    int done = 0;
-    if (S >= 8) {
-        unsigned dm = __ballot_sync(kFull, dif);
-        while (dm) {
-            const int src = __ffs(dm) - 1;
-            dm &= dm - 1;
-            const RayState q = shfl_ray(fe, src);
-            const int32_t qi = __shfl_sync(kFull, ti, src);
-            const Tri T = load_tri(tris, qi);
-            for (int s0 = 0; s0 < S; s0 += 32) {
-                const int s = s0 + lane_id();
-                bool ok = false;
-                int64_t off = 0;
-                float inten = 0.f;
-                if (s < S) ok = sample_of(sp, q, T, s, off, inten);
-                accumulate_warp(sp, ok, off, inten);
-                done += ok ? 1 : 0;
-            }
-        }
-    } else if (dif) {
-        const Tri T = load_tri(tris, ti);
-        for (int s = 0; s < S; ++s) {
-            int64_t off;
-            float inten;
-            if (sample_of(sp, fe, T, s, off, inten)) {
-                accumulate_one(sp, off, inten);
-                ++done;
-            }
-        }
-    }
-    return done;
-}
 
 __device__ __forceinline__ void add_stats(splat_trace_stats_t* st, int diffuse, int samples) {
     if (!st) return;
@@ -270,19 +168,30 @@ cudaError_t launch_evolve_plugin(const EvolveArgs& a, int64_t cap, int sm_count,
 __global__ void __launch_bounds__(kEvolveThreads) evolve_aos_kernel(splat_adray_t* rays, int64_t n,
                                                                     const int32_t* __restrict__ hit_idx,
                                                                     const float* __restrict__ rndm, EvolveArgs A) {
+    __shared__ AosTile s_tile[kEvolveThreads / 32];
+    AosTile& tile = s_tile[threadIdx.x >> 5];
     const bool quirks = A.quirks != 0;
-    for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < n; k += (int64_t)gridDim.x * blockDim.x) {
-        splat_adray_t& a = rays[k];
-        if (a.status != kStatusActive) continue;
-        const RayState r = ray_from_aos(a);
-        const EvolveView v{A.tris, A.n_tris, A.err, A.first_diffuse, A.material, A.seed, A.bounce,
-                           rndm ? rndm[k] : A.force_rand, quirks, false};
-        RayState o;
-        int32_t ih;
-        const int fate = evolve_one<false>(r, hit_idx[k], (uint32_t)k, v, o, ih);
-        if (fate == kFateKeep) ray_to_aos(a, o, kStatusActive);
-        else if (fate == kFateDiffuse) a.status = (uint8_t)kStatusDiffuse;
-        else if (fate == kFateInfinity) a.status = (uint8_t)kStatusInfinity;
+    const int lane = lane_id();
+    for (int64_t base = blockIdx.x * (int64_t)blockDim.x + threadIdx.x - lane; base < n;
+         base += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t k = base + lane;
+        // the status first: a warp of retired rays moves nothing
+        const bool act = k < n && rays[k].status == kStatusActive;
+        if (!__any_sync(kFull, act)) continue;
+        aos_tile_load(tile, rays, base, n);
+        if (act) {
+            splat_adray_t& a = aos_tile_ray(tile);
+            const RayState r = ray_from_aos(a);
+            const EvolveView v{A.tris, A.n_tris, A.err, A.first_diffuse, A.material, A.seed, A.bounce,
+                               rndm ? rndm[k] : A.force_rand, quirks, false};
+            RayState o;
+            int32_t ih;
+            const int fate = evolve_one<false>(r, hit_idx[k], (uint32_t)k, v, o, ih);
+            if (fate == kFateKeep) ray_to_aos(a, o, kStatusActive);
+            else if (fate == kFateDiffuse) a.status = (uint8_t)kStatusDiffuse;
+            else if (fate == kFateInfinity) a.status = (uint8_t)kStatusInfinity;
+        }
+        aos_tile_store(tile, rays, base, n);
     }
 }
 
@@ -341,31 +250,96 @@ cudaError_t launch_partition(splat_adray_t* rays, int64_t n, splat_adray_t* swap
 }
 
 // continuum_light_map2! on the caller's AoS rays: final_evolution in place,
-// then the splat.
-__global__ void __launch_bounds__(kEvolveThreads) light_map_kernel(splat_adray_t* rays, int64_t n,
-                                                                   const int32_t* __restrict__ hit_idx,
-                                                                   const splat_ftri_t* __restrict__ tris,
-                                                                   int64_t n_tris, int32_t* err, SplatParams sp) {
+// then the splat, one lane per diffuse ray walking all its planes as in
+// splat_kernel.  The block's diffuse rays are compacted through shared memory
+// between the two (their records' tile slots are reused: a ray's float planes
+// and triangle index, 28 words of its 34), so warps splat with all lanes
+// busy.  What it was bound by before: one ray at a time per warp, its 27
+// values and triangle broadcast to the lanes that held its samples.  2^18
+// rays, 12 planes, 2 x 2 offsets: 311.7 -> 154.3 us (ncu, one GB300).
+__global__ void __launch_bounds__(kEvolveThreads, 2) light_map_kernel(splat_adray_t* rays, int64_t n,
+                                                                      const int32_t* __restrict__ hit_idx,
+                                                                      const splat_ftri_t* __restrict__ tris,
+                                                                      int64_t n_tris, int32_t* err, SplatParams sp) {
+    constexpr int kWarps = kEvolveThreads / 32;
+    __shared__ AosTile s_tile[kWarps];
+    __shared__ int s_cnt[kWarps];
+    float* pool = reinterpret_cast<float*>(s_tile);  // [plane][kEvolveThreads], kPlanes + 1 planes
+    static_assert(sizeof(s_tile) >= sizeof(float) * (kPlanes + 1) * kEvolveThreads, "pool fits the tiles");
+    const int lane = lane_id(), wid = threadIdx.x >> 5;
+    AosTile& tile = s_tile[wid];
+    const int planes = sp.n_lambda > 0 ? sp.n_lambda : 1;
     for (int64_t base = (int64_t)blockIdx.x * kEvolveThreads; base < n; base += (int64_t)gridDim.x * kEvolveThreads) {
-        const int64_t k = base + threadIdx.x;
+        const int64_t wbase = base + 32 * wid, k = wbase + lane;
         bool dif = false;
         RayState o;
         int32_t ih = 1;
-        if (k < n && rays[k].status == kStatusDiffuse) {
-            const int32_t i = hit_idx[k];
-            if (i >= 1 && i <= n_tris) {
-                const RayState r = ray_from_aos(rays[k]);
-                const Tri T = load_tri(tris, i);
-                HitDerivs h;
-                ih = get_hit_ad(r, i, T, h);
-                final_evolution(r, h, ih, o);
-                ray_to_aos(rays[k], o, kStatusDiffuse);
-                dif = true;
-            } else {
-                atomicOr(err, 16);
+        const bool want = k < n && rays[k].status == kStatusDiffuse;
+        if (__any_sync(kFull, want)) {
+            aos_tile_load(tile, rays, wbase, n);
+            if (want) {
+                const int32_t i = hit_idx[k];
+                if (i >= 1 && i <= n_tris) {
+                    splat_adray_t& a = aos_tile_ray(tile);
+                    const RayState r = ray_from_aos(a);
+                    const Tri T = load_tri(tris, i);
+                    HitDerivs h;
+                    ih = get_hit_ad(r, i, T, h);
+                    final_evolution(r, h, ih, o);
+                    ray_to_aos(a, o, kStatusDiffuse);
+                    dif = true;
+                } else {
+                    atomicOr(err, 16);
+                }
             }
+            aos_tile_store(tile, rays, wbase, n);
         }
-        (void)splat_warp(sp, tris, dif, o, ih);
+        const unsigned db = __ballot_sync(kFull, dif);
+        if (lane == 0) s_cnt[wid] = __popc(db);
+        __syncthreads();  // every warp is done with its tile
+        int before = 0, total = 0;
+#pragma unroll
+        for (int w = 0; w < kWarps; ++w) {
+            const int c = s_cnt[w];
+            before += w < wid ? c : 0;
+            total += c;
+        }
+        const RaySoA q{pool, nullptr, nullptr, nullptr, kEvolveThreads};
+        if (dif) {
+            const int p = before + __popc(db & ((1u << lane) - 1u));
+            st3(q.f, q.cap, 0, p, o.pos);
+            st3(q.f, q.cap, 3, p, o.dir);
+            st3(q.f, q.cap, 6, p, o.dpl);
+            st3(q.f, q.cap, 9, p, o.dpx);
+            st3(q.f, q.cap, 12, p, o.dpy);
+            st3(q.f, q.cap, 15, p, o.ddl);
+            st3(q.f, q.cap, 18, p, o.ddx);
+            st3(q.f, q.cap, 21, p, o.ddy);
+            q.f[24 * q.cap + p] = o.lam;
+            q.f[25 * q.cap + p] = o.x;
+            q.f[26 * q.cap + p] = o.y;
+            q.f[27 * q.cap + p] = __int_as_float(ih);
+        }
+        __syncthreads();
+        if ((int)threadIdx.x < total) {
+            const int p = threadIdx.x;
+            RayState s;
+            s.pos = ld3(q.f, q.cap, 0, p);
+            s.dir = ld3(q.f, q.cap, 3, p);
+            s.dpl = ld3(q.f, q.cap, 6, p);
+            s.dpx = ld3(q.f, q.cap, 9, p);
+            s.dpy = ld3(q.f, q.cap, 12, p);
+            s.ddl = ld3(q.f, q.cap, 15, p);
+            s.ddx = ld3(q.f, q.cap, 18, p);
+            s.ddy = ld3(q.f, q.cap, 21, p);
+            s.lam = q.f[24 * q.cap + p];
+            s.x = q.f[25 * q.cap + p];
+            s.y = q.f[26 * q.cap + p];
+            const Tri T = load_tri(tris, __float_as_int(q.f[27 * q.cap + p]));
+            const TriUV quv = tri_uv(T);
+            for (int il = 0; il < planes; ++il) (void)splat_ray_plane(sp, s, T, quv, il);
+        }
+        __syncthreads();  // the tiles are free again
     }
 }
 
@@ -485,14 +459,23 @@ __global__ void generate_soa_kernel(GenParams g, int64_t n, RaySoA out, int64_t*
     }
 }
 
-__global__ void generate_aos_kernel(GenParams g, int64_t n, splat_adray_t* out) {
-    for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < n; k += (int64_t)gridDim.x * blockDim.x) {
-        const RayState r = gen_ray(g, g.ray_begin + k);
-        splat_adray_t a;
-        memset(&a, 0, sizeof(a));
-        ray_to_aos(a, r, kStatusActive);
-        a.dest = 0;
-        out[k] = a;
+__global__ void __launch_bounds__(256) generate_aos_kernel(GenParams g, int64_t n, splat_adray_t* out) {
+    __shared__ AosTile s_tile[256 / 32];
+    AosTile& tile = s_tile[threadIdx.x >> 5];
+    const int lane = lane_id();
+    for (int64_t base = blockIdx.x * (int64_t)blockDim.x + threadIdx.x - lane; base < n;
+         base += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t k = base + lane;
+        if (k < n) {
+            const RayState r = gen_ray(g, g.ray_begin + k);
+            splat_adray_t a;
+            memset(&a, 0, sizeof(a));
+            ray_to_aos(a, r, kStatusActive);
+            a.dest = 0;
+            aos_tile_ray(tile) = a;
+        }
+        aos_tile_store(tile, out, base, n);
+        __syncwarp();
     }
 }
 
@@ -511,18 +494,25 @@ cudaError_t launch_generate_aos(const GenParams& g, int64_t n, splat_adray_t* ou
 }
 
 // active AoS rays -> SoA (id = slot), compacted with one atomic per warp
-__global__ void aos_to_soa_kernel(const splat_adray_t* in, int64_t n, RaySoA out, int64_t* d_count) {
-    for (int64_t base = (int64_t)blockIdx.x * blockDim.x; base < n; base += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t k = base + threadIdx.x;
-        const bool act = k < n && in[k].status == kStatusActive;
+__global__ void __launch_bounds__(256) aos_to_soa_kernel(const splat_adray_t* in, int64_t n, RaySoA out,
+                                                         int64_t* d_count) {
+    __shared__ AosTile s_tile[256 / 32];
+    AosTile& tile = s_tile[threadIdx.x >> 5];
+    const int lane = lane_id();
+    for (int64_t base = blockIdx.x * (int64_t)blockDim.x + threadIdx.x - lane; base < n;
+         base += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t k = base + lane;
+        aos_tile_load(tile, in, base, n);
+        const splat_adray_t& a = aos_tile_ray(tile);
+        const bool act = k < n && a.status == kStatusActive;
         const unsigned b = __ballot_sync(kFull, act);
         unsigned long long wbase = 0;
-        if (lane_id() == 0 && b)
+        if (lane == 0 && b)
             wbase = atomicAdd(reinterpret_cast<unsigned long long*>(d_count), (unsigned long long)__popc(b));
         wbase = __shfl_sync(kFull, wbase, 0);
         if (act) {
-            const int64_t pos = (int64_t)wbase + __popc(b & ((1u << lane_id()) - 1u));
-            store_ray(out, pos, ray_from_aos(in[k]), (uint32_t)k);
+            const int64_t pos = (int64_t)wbase + __popc(b & ((1u << lane) - 1u));
+            store_ray(out, pos, ray_from_aos(a), (uint32_t)k);
         }
     }
 }
