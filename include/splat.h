@@ -280,7 +280,7 @@ splat_status_t splat_evolve(const splat_scene_t* scene, splat_adray_t* d_rays, i
  * called at src/tracer.jl:263): the ACTIVE rays move to the front of d_rays,
  * in no particular order (the reference's is not stable either), and their
  * count is written to the device int64 *d_n_active -- it is not read back.
- * Workspace: splat_partition_workspace_size(n_rays) bytes (the swap array). */
+ * Workspace: splat_partition_workspace_size(n_rays) bytes. */
 size_t splat_partition_workspace_size(int64_t n_rays);
 splat_status_t splat_partition(splat_adray_t* d_rays, int64_t n_rays, int64_t* d_n_active, void* d_workspace,
                                size_t workspace_bytes, void* stream);

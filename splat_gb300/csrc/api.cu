@@ -690,12 +690,10 @@ splat_status_t splat_partition(splat_adray_t* d_rays, int64_t n_rays, int64_t* d
     if (reinterpret_cast<uintptr_t>(d_workspace) % 16) return fail(SPLAT_ERR_INVALID, "partition: workspace not 16-byte aligned");
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     int64_t* counts = reinterpret_cast<int64_t*>(d_workspace);
-    splat_adray_t* swap = reinterpret_cast<splat_adray_t*>(static_cast<char*>(d_workspace) + kAlign);
-    {
-        ProfScope ps(SPLAT_KERNEL_AUX, st);
-        SPLAT_CUDA(launch_partition(d_rays, n_rays, swap, counts, sm_count_current(), st), "partition");
-    }
-    SPLAT_CUDA(cudaMemcpyAsync(d_n_active, counts, sizeof(int64_t), cudaMemcpyDeviceToDevice, st), "partition count");
+    int64_t* list = reinterpret_cast<int64_t*>(static_cast<char*>(d_workspace) + kAlign);
+    static_assert(2 * sizeof(int64_t) <= sizeof(splat_adray_t), "both lists fit the workspace");
+    ProfScope ps(SPLAT_KERNEL_AUX, st);
+    SPLAT_CUDA(launch_partition(d_rays, n_rays, counts, list, d_n_active, sm_count_current(), st), "partition");
     return SPLAT_OK;
 }
 

@@ -251,9 +251,9 @@ cudaError_t launch_evolve_plugin(const EvolveArgs& a, int64_t cap, int sm_count,
 // one evolve_ray broadcast on AoS rays (rndm: per-ray draws or null)
 cudaError_t launch_evolve_aos(splat_adray_t* rays, int64_t n, const int32_t* hit_idx, const float* rndm,
                               const EvolveArgs& a, int sm_count, cudaStream_t s);
-// partition!: ACTIVE rays first via swap; counts[0] = their number (3 int64)
-cudaError_t launch_partition(splat_adray_t* rays, int64_t n, splat_adray_t* swap, int64_t* counts, int sm_count,
-                             cudaStream_t s);
+// partition!: ACTIVE rays first, in place; scratch: counts (3 int64), list (2 n int64)
+cudaError_t launch_partition(splat_adray_t* rays, int64_t n, int64_t* counts, int64_t* list, int64_t* d_n_active,
+                             int sm_count, cudaStream_t s);
 cudaError_t launch_light_map(splat_adray_t* rays, int64_t n, const int32_t* hit_idx, const splat_ftri_t* tris,
                              int64_t n_tris, int32_t* err, const SplatParams& sp, int sm_count, cudaStream_t s);
 // camera pass (shade.cu)
