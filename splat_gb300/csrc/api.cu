@@ -626,6 +626,7 @@ splat_status_t splat_run_evolution(const splat_scene_t* scene, int32_t hitter, s
     for (int32_t b = 1; b <= depth; ++b) {
         RaySrc src{cur.f, cur.ignore, cur.cap, nullptr, &w.counts[b - 1], 0,
                    reinterpret_cast<unsigned long long*>(&w.counts[kFetchBase + b]), packet_for(b)};
+        src.few = b > 1 ? 1 : 0;
         splat_status_t rc = hit_any(scene, hitter, src, n_rays, w.hit, nullptr, w.tmp, st);
         if (rc != SPLAT_OK) return rc;
         ea.in = cur;
@@ -806,8 +807,14 @@ static int64_t grid_rays(const splat_trace_params_t* P) {
 // on stream st: generate, depth x {hit, evolve (+ compaction, diffuse
 // queue)}, the splat (segments on a side stream), the statistics.  The map
 // and d_stats were cleared by the caller; statistics accumulate.
+// alone: a small step in one range.  Its later bounces may leave few rays, and
+// their hit launches prepare for that (RaySrc::few).  A large step's do not:
+// beside the other range and the splats its last bounces' latency is hidden
+// already, and a second launch, whose shared memory the running kernels' SMs
+// must first make room for, costs more (2^20 rays: 1.36 -> 1.40 ms).
 static splat_status_t trace_part(const splat_scene_t* scene, const splat_trace_params_t* P, void* d_map, Work w,
-                                 int64_t rb, int64_t cnt, splat_trace_stats_t* d_stats, cudaStream_t st, int sm) {
+                                 int64_t rb, int64_t cnt, splat_trace_stats_t* d_stats, cudaStream_t st, int sm,
+                                 bool alone) {
     GenParams g;
     g.light = P->light;
     g.upscale = P->upscale;
@@ -849,6 +856,7 @@ static splat_status_t trace_part(const splat_scene_t* scene, const splat_trace_p
     for (int32_t b = 1; b <= P->depth; ++b) {
         RaySrc src{cur.f, cur.ignore, cur.cap, nullptr, &w.counts[b - 1], 0,
                    reinterpret_cast<unsigned long long*>(&w.counts[kFetchBase + b]), packet_for(b)};
+        src.few = b > 1 && alone ? 1 : 0;
         {
             // the first bounce's rays are the light grid's columns in order
             // (the range starts on a column): packet warps take 8 x 4 tiles
@@ -2006,6 +2014,7 @@ splat_status_t splat_render_camera_after(const splat_scene_t* scene, const splat
     for (int32_t b = 1; b <= P->depth; ++b) {
         RaySrc src{cur.f, cur.ignore, cur.cap, nullptr, &w.counts[b - 1], 0,
                    reinterpret_cast<unsigned long long*>(&w.counts[kFetchBase + b]), packet_for(b)};
+        src.few = b > 1 && cnt < kSplitMinRays ? 1 : 0;
         // camera rays are the sub-sample grid's columns in order: first-bounce
         // packets take 8 x 4 tiles of it
         if (b == 1 && ch <= (int64_t)kGridTileMaxRows) src.tile_h = (int32_t)ch;

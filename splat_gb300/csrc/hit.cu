@@ -622,6 +622,7 @@ __global__ void __launch_bounds__(kBvhThreads) hit_bvh4_kernel(RaySrc src, Bvh4V
                                                                int32_t* __restrict__ hit_idx,
                                                                float* __restrict__ hit_t, int32_t* err) {
     const int64_t n = src.d_count ? *src.d_count : src.n;
+    if (src.few && n <= kGroupRays) return;  // the group kernel's
     int2 stack[kBvhStack];
     WorkCount wc{0u, 0u, 0u};
     uint32_t rays = 0;
@@ -638,6 +639,25 @@ __global__ void __launch_bounds__(kBvhThreads) hit_bvh4_kernel(RaySrc src, Bvh4V
     if (COUNT) flush_work(wc, rays);
 }
 
+
+// Few rays: a warp or eight lanes a ray (bvh4_group_loop).
+template <bool AOS>
+__global__ void __launch_bounds__(kBvhThreads) hit_bvh4_group_kernel(RaySrc src, Bvh4View bvh,
+                                                                     int32_t* __restrict__ hit_idx,
+                                                                     float* __restrict__ hit_t) {
+    __shared__ int2 s_stack[kBvhThreads / 32][kGroupStackWarp];
+    const int64_t n = src.d_count ? *src.d_count : src.n;
+    if (n > kGroupRays) return;
+    auto ray_of = [&](int64_t kk) { return src.perm ? (int64_t)src.perm[kk] : kk; };
+    bvh4_groups(
+        n, src.fetch, s_stack[threadIdx.x >> 5], [&](int64_t kk) { return load_hit_ray<AOS>(src, ray_of(kk)); },
+        [&](int64_t) { return bvh; },
+        [&](int64_t kk, float best, int32_t bi) {
+            const int64_t k = ray_of(kk);
+            hit_idx[k] = bi;
+            if (hit_t) hit_t[k] = best;
+        });
+}
 
 // The per-ray form with finished lanes refilled from the work counter.
 template <bool AOS>
@@ -769,10 +789,31 @@ cudaError_t launch_hit_bvh4(const RaySrc& rays, int64_t cap, const Bvh4View& bvh
         prefer_l1(hit_bvh_kernel<false>);
         configured = true;
     }
-    if (g_tune[SPLAT_TUNE_COUNT_WORK])
+    if (g_tune[SPLAT_TUNE_COUNT_WORK]) {
         launch_bvh4_form<true>(rays, cap, bvh, hit_idx, hit_t, err, sm_count, s);
-    else
-        launch_bvh4_form<false>(rays, cap, bvh, hit_idx, hit_t, err, sm_count, s);
+        ++g_launches;
+        return cudaGetLastError();
+    }
+    // Few rays go to the group kernel.  Their number is known here when it is
+    // the launch's bound; otherwise, where few are likely (few), both kernels
+    // are launched and the count on the device picks the one that works.
+    // Packet and refill forms that were asked for by their knobs stay.
+    const bool groups = g_tune[SPLAT_TUNE_BVH_REFILL] == 0 && g_tune[SPLAT_TUNE_BVH_PACKET] <= 1;
+    RaySrc src = rays;
+    src.few = groups && rays.few && rays.packet == 0 ? 1 : 0;
+    const bool only = groups && cap <= kGroupRays;
+    if (only || src.few) {
+        const int64_t lanes = cap <= kGroupWarpRays ? 32 * cap : std::max(32 * kGroupWarpRays, 8 * std::min(cap, kGroupRays));
+        const int grid = resident_grid(reinterpret_cast<const void*>(hit_bvh4_group_kernel<false>), lanes, sm_count,
+                                       kBvhThreads, 256);
+        if (rays.aos)
+            hit_bvh4_group_kernel<true><<<grid, kBvhThreads, 0, s>>>(src, bvh, hit_idx, hit_t);
+        else
+            hit_bvh4_group_kernel<false><<<grid, kBvhThreads, 0, s>>>(src, bvh, hit_idx, hit_t);
+        ++g_launches;
+        if (only) return cudaGetLastError();
+    }
+    launch_bvh4_form<false>(src, cap, bvh, hit_idx, hit_t, err, sm_count, s);
     ++g_launches;
     return cudaGetLastError();
 }

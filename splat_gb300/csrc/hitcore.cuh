@@ -483,6 +483,171 @@ __device__ __forceinline__ void bvh4_closest_packet(const HitRay& r, bool valid,
     bi_out = bi;
 }
 
+// Group traversal: G lanes (a power of two) walk one ray through its
+// four-wide BVH, each lane taking one entry -- a node or a leaf -- off the
+// group's stack per step; children a lane enters go back onto the stack, and
+// the group keeps one best hit.  A step takes the entries on top, so the walk
+// stays depth first in chunks of G.  The boxes entered are a superset of the
+// one-lane walk's (an entry is dropped only when its distance is beyond the
+// best hit), so the lexicographic (t, index) minimum is the same.  The chain
+// of dependent node loads shrinks from the ray's visits to about the tree's
+// depth plus visits / G steps, at the price of more visits: for launches with
+// too few rays to fill the GPU, where one hard ray's chain is the launch.
+// stack: kGroupStack<G> entries of shared memory per group.  A step takes no
+// more entries than the room above leaves space for (three net pushes each),
+// and with less than that it takes one, which needs at most kBvhStack more
+// entries (the builder's bound on three per level), so the stack cannot
+// overflow.
+//
+// Measured on one GB300 (us a next_hit call, scattered rays; one lane a ray /
+// eight / thirty-two; a call's host work is about 15 us of each):
+//   rays                        1,000        4,000        10,000       20,000       40,000       80,000
+//   displaced sphere, 81,922    42/19/19     58/21/17     67/28/28     67/34/47     77/53/84     87/87/155
+//   turned sponge, 96,012       24/22/18     27/24/20     28/27/30     29/32/48     31/47/80     36/78/143
+// Hence a warp a ray up to kGroupWarpRays, eight lanes up to kGroupRays.
+template <int G>
+constexpr int kGroupStack = kBvhStack + (G == 32 ? 448 : 64);
+constexpr int kGroupStackWarp = kGroupStack<32>;
+static_assert(kGroupStackWarp >= 4 * kGroupStack<8>, "one warp's stacks");
+constexpr int64_t kGroupWarpRays = 4096;
+constexpr int64_t kGroupRays = 16384;
+
+// load(k): ray k; view(k): the BVH it is traced in; store(k, t, index).
+// Groups take rays off the work counter, or stride statically without one.
+template <int G, class Load, class View, class Store>
+__device__ __forceinline__ void bvh4_group_loop(int64_t n, unsigned long long* fetch, int2* stack, const Load& load,
+                                                const View& view, const Store& store) {
+    static_assert(G == 8 || G == 32, "group size");
+    const float kInf = __int_as_float(0x7f800000);
+    const int lane = threadIdx.x & 31, gl = lane & (G - 1), g0 = lane & ~(G - 1);
+    const unsigned gmask = G == 32 ? 0xffffffffu : ((1u << (G & 31)) - 1u) << g0;
+    const unsigned below = (1u << lane) - 1u;
+    const int64_t groups = (int64_t)gridDim.x * (blockDim.x / G);
+    int64_t next = (int64_t)blockIdx.x * (blockDim.x / G) + threadIdx.x / G;
+    HitRay r{};
+    SlabRay sr{};
+    Bvh4View bvh{};
+    float best = kInf;
+    int32_t bi = 1;
+    int sp = 0;
+    int64_t k = -1;  // the group's ray; -1: none
+    bool more = true;
+    while (true) {
+        if (sp == 0) {  // group-uniform
+            if (k >= 0 && gl == 0) store(k, best, bi);
+            k = -1;
+        }
+        // idle groups take the next rays, one atomic per warp
+        const unsigned idle = __ballot_sync(0xffffffffu, k < 0 && gl == 0);
+        if (idle && more) {
+            unsigned long long base = 0;
+            if (fetch) {
+                if (lane == 0) base = atomicAdd(fetch, (unsigned long long)__popc(idle));
+                base = __shfl_sync(0xffffffffu, base, 0);
+                if (base + (unsigned long long)__popc(idle) >= (unsigned long long)n) more = false;
+            }
+            if (k < 0) {
+                int64_t kk;
+                if (fetch) {
+                    kk = (int64_t)base + __popc(idle & ((1u << g0) - 1u));
+                } else {
+                    kk = next;
+                    next += groups;
+                }
+                if (kk < n) {
+                    k = kk;
+                    r = load(k);
+                    bvh = view(k);
+                    sr = slab_ray(r, bvh.nodes);
+                    best = kInf;
+                    bi = 1;
+                    sp = 1;
+                    if (gl == 0) stack[0] = make_int2(0, 0);
+                }
+            }
+            if (!fetch) more = __any_sync(0xffffffffu, next < n);
+        }
+        if (!more && __all_sync(0xffffffffu, k < 0)) break;
+        __syncwarp();
+        const int room = (kGroupStack<G> - kBvhStack - sp) / 3;
+        const int take = min(min(sp, G), max(room, 1));
+        const bool mine = gl < take;
+        sp -= take;
+        int ref = 0;
+        bool go = false;
+        if (mine) {
+            const int2 e = stack[sp + gl];
+            ref = e.x;
+            go = __int_as_float(e.y) <= best;
+        }
+        bool h[4] = {false, false, false, false};
+        float tmin[4] = {0.f, 0.f, 0.f, 0.f};
+        int4 c = make_int4(0, 0, 0, 0);
+        float lb = best;
+        int32_t li = bi;
+        if (go && ref >= 0) {
+            const Bvh4Node* nd = bvh.nodes + ref;
+            c = __ldg(&nd->c);
+            float tmax[4];
+            node4_slabs(nd, sr.ix, sr.iy, sr.iz, sr.oix, sr.oiy, sr.oiz, tmin, tmax);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) h[i] = (tmin[i] <= tmax[i]) & (tmin[i] <= best);
+        } else if (go) {
+            const int enc = ~ref;
+            const int first = enc >> 4;
+            const int count = (enc & 15) + 1;
+            for (int j = 0; j < count; ++j) {
+                const TriHit* t3 = bvh.tris + first + j;
+                float num, den;
+                if (!tri_candidate(__ldg(&t3->n_nv), r, lb, num, den)) continue;
+                const float4 q1 = __ldg(&t3->a_idx);
+                const int32_t idx = __float_as_int(q1.w);
+                bool inside;
+                const float t = tri_t_from(num, den, q1, __ldg(&t3->e0), __ldg(&t3->e1), __ldg(&t3->inv), r, inside);
+                if (inside & (t > 0.0f) & (idx != r.ig) & ((t < lb) | ((t == lb) & (idx < li)))) {
+                    lb = t;
+                    li = idx;
+                }
+            }
+        }
+        __syncwarp();  // the entries taken have been read
+        if (__any_sync(0xffffffffu, (lb < best) | (li != bi))) {
+            // the group's smallest (t, index); t >= 0, so its bits order as it
+#pragma unroll
+            for (int o = G / 2; o; o >>= 1) {
+                const float ot = __shfl_xor_sync(0xffffffffu, lb, o);
+                const int32_t oi = __shfl_xor_sync(0xffffffffu, li, o);
+                if ((ot < lb) | ((ot == lb) & (oi < li))) {
+                    lb = ot;
+                    li = oi;
+                }
+            }
+            best = lb;
+            bi = li;
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const unsigned m = __ballot_sync(0xffffffffu, h[i]) & gmask;
+            if (h[i]) {
+                const int ci = i == 0 ? c.x : (i == 1 ? c.y : (i == 2 ? c.z : c.w));
+                stack[sp + __popc(m & below)] = make_int2(ci, __float_as_int(tmin[i]));
+            }
+            sp += __popc(m);
+        }
+    }
+}
+
+// n <= kGroupRays rays by the group size that suits their number; stack: the
+// warp's kGroupStackWarp entries.
+template <class Load, class View, class Store>
+__device__ __forceinline__ void bvh4_groups(int64_t n, unsigned long long* fetch, int2* stack, const Load& load,
+                                            const View& view, const Store& store) {
+    if (n <= kGroupWarpRays)
+        bvh4_group_loop<32>(n, fetch, stack, load, view, store);
+    else
+        bvh4_group_loop<8>(n, fetch, stack + ((threadIdx.x & 31) >> 3) * kGroupStack<8>, load, view, store);
+}
+
 // Spread of a warp's rays, max over axes of (max - min) of a coordinate.
 __device__ __forceinline__ float warp_spread(float a, float b, float c) {
     float m = 0.0f;

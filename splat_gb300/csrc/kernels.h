@@ -31,6 +31,8 @@ struct RaySrc {
                                // go to the ray's own index
     int32_t tile_h;            // packet kernels, no perm: rays are a light grid of tile_h rows in column-major
                                // order; warps take 8 x 4 tiles of it (0: in order)
+    int32_t few;               // the count on the device may be far below the launch's bound (later bounces):
+                               // four-wide BVH launches prepare for kGroupRays rays or less
 };
 
 // Which traversal a warp of four-wide BVH rays takes, from

@@ -66,6 +66,9 @@ def test_hits_equal_brute_force_in_any_frame(turn):
                 hit, t = tracer.next_hit(scene, hitter, d_rays, with_t=True)
                 assert torch.equal(hit, ref), (what, hitter, packet)
                 assert torch.equal(t.view(torch.int32), tref.view(torch.int32)), (what, hitter, packet)
+                # enough rays for one lane a ray
+                hit = tracer.next_hit(scene, hitter, d_rays.repeat(5))
+                assert torch.equal(hit, ref.repeat(5)), (what, hitter, packet, "many")
         finally:
             L.check(lib.splat_set_tuning(L.TUNE_BVH_PACKET, old))
 
