@@ -81,8 +81,11 @@ __global__ void __launch_bounds__(kEvolveThreads) evolve_kernel(EvolveArgs A) {
             keep = fate == kFateKeep;
             dif = fate == kFateDiffuse;
             sky = SKY && fate == kFateInfinity;
-            if (!TRACE && fate == kFateDiffuse) ray_to_aos(A.aos[id], r, kStatusDiffuse);
-            if (!TRACE && fate == kFateInfinity) ray_to_aos(A.aos[id], r, kStatusInfinity);
+            if (!TRACE && fate != kFateKeep) {
+                // the state written back is the one this hit was found for
+                ray_to_aos(A.aos[id], r, fate == kFateDiffuse ? kStatusDiffuse : kStatusInfinity);
+                A.aos_hit[id] = A.hit_idx[k];
+            }
         }
         // compaction of the survivors (and, tracing, of the diffuse rays into
         // the splat queue and of the escaped ones into the sky queue): ballot
@@ -526,9 +529,10 @@ cudaError_t launch_generate_aos(const GenParams& g, int64_t n, splat_adray_t* ou
     return cudaGetLastError();
 }
 
-// active AoS rays -> SoA (id = slot), compacted with one atomic per warp
+// AoS rays -> SoA (id = slot), the active ones to out and the others to idle,
+// compacted with one atomic per warp and target
 __global__ void __launch_bounds__(256) aos_to_soa_kernel(const splat_adray_t* in, int64_t n, RaySoA out,
-                                                         int64_t* d_count) {
+                                                         int64_t* d_count, RaySoA idle, int64_t* d_idle) {
     __shared__ AosTile s_tile[256 / 32];
     AosTile& tile = s_tile[threadIdx.x >> 5];
     const int lane = lane_id();
@@ -538,34 +542,64 @@ __global__ void __launch_bounds__(256) aos_to_soa_kernel(const splat_adray_t* in
         aos_tile_load(tile, in, base, n);
         const splat_adray_t& a = aos_tile_ray(tile);
         const bool act = k < n && a.status == kStatusActive;
+        const unsigned valid = __ballot_sync(kFull, k < n);
         const unsigned b = __ballot_sync(kFull, act);
-        unsigned long long wbase = 0;
+        unsigned long long wbase = 0, ibase = 0;
         if (lane == 0 && b)
             wbase = atomicAdd(reinterpret_cast<unsigned long long*>(d_count), (unsigned long long)__popc(b));
+        if (lane == 0 && b != valid)
+            ibase = atomicAdd(reinterpret_cast<unsigned long long*>(d_idle), (unsigned long long)__popc(valid & ~b));
         wbase = __shfl_sync(kFull, wbase, 0);
-        if (act) {
-            const int64_t pos = (int64_t)wbase + __popc(b & ((1u << lane) - 1u));
-            store_ray(out, pos, ray_from_aos(a), (uint32_t)k);
-        }
+        ibase = __shfl_sync(kFull, ibase, 0);
+        const unsigned below = (1u << lane) - 1u;
+        if (act)
+            store_ray(out, (int64_t)wbase + __popc(b & below), ray_from_aos(a), (uint32_t)k);
+        else if (k < n)
+            store_ray(idle, (int64_t)ibase + __popc(valid & ~b & below), ray_from_aos(a), (uint32_t)k);
     }
 }
 
-__global__ void soa_to_aos_kernel(RaySoA in, const int64_t* d_count, splat_adray_t* out, int status) {
-    const int64_t n = *d_count;
-    for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < n; k += (int64_t)gridDim.x * blockDim.x)
-        ray_to_aos(out[in.id[k]], load_ray(in, k), status);
+__global__ void append_idle_kernel(RaySoA rays, const int64_t* d_count, RaySoA idle, const int64_t* d_idle,
+                                   int64_t* d_total) {
+    const int64_t m = *d_count, z = *d_idle;
+    if (blockIdx.x == 0 && threadIdx.x == 0) *d_total = m + z;
+    for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < z; j += (int64_t)gridDim.x * blockDim.x) {
+        st3(rays.f, rays.cap, 0, m + j, ld3(idle.f, idle.cap, 0, j));
+        st3(rays.f, rays.cap, 3, m + j, ld3(idle.f, idle.cap, 3, j));
+        rays.ignore[m + j] = idle.ignore[j];
+        rays.id[m + j] = idle.id[j];
+    }
 }
 
-cudaError_t launch_aos_to_soa(const splat_adray_t* in, int64_t n, RaySoA out, int64_t* d_count, cudaStream_t s) {
+__global__ void soa_to_aos_kernel(RaySoA in, const int64_t* d_count, const int64_t* d_total,
+                                  const int32_t* __restrict__ hit, splat_adray_t* out, int32_t* hit_out, int status) {
+    const int64_t m = *d_count, n = *d_total;
+    for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < n; k += (int64_t)gridDim.x * blockDim.x) {
+        const uint32_t id = in.id[k];
+        hit_out[id] = hit[k];
+        if (k < m) ray_to_aos(out[id], load_ray(in, k), status);
+    }
+}
+
+cudaError_t launch_aos_to_soa(const splat_adray_t* in, int64_t n, RaySoA out, int64_t* d_count, RaySoA idle,
+                              int64_t* d_idle, cudaStream_t s) {
     if (n <= 0) return cudaSuccess;
-    aos_to_soa_kernel<<<evolve_grid(n, 152), 256, 0, s>>>(in, n, out, d_count);
+    aos_to_soa_kernel<<<evolve_grid(n, 152), 256, 0, s>>>(in, n, out, d_count, idle, d_idle);
     ++g_launches;
     return cudaGetLastError();
 }
 
-cudaError_t launch_soa_to_aos(RaySoA in, const int64_t* d_count, splat_adray_t* out, int status, cudaStream_t s) {
+cudaError_t launch_append_idle(RaySoA rays, const int64_t* d_count, RaySoA idle, const int64_t* d_idle,
+                               int64_t* d_total, int sm_count, cudaStream_t s) {
+    append_idle_kernel<<<sm_count, 256, 0, s>>>(rays, d_count, idle, d_idle, d_total);
+    ++g_launches;
+    return cudaGetLastError();
+}
+
+cudaError_t launch_soa_to_aos(RaySoA in, const int64_t* d_count, const int64_t* d_total, const int32_t* hit,
+                              splat_adray_t* out, int32_t* hit_out, int status, cudaStream_t s) {
     if (in.cap <= 0) return cudaSuccess;
-    soa_to_aos_kernel<<<evolve_grid(in.cap, 152), 256, 0, s>>>(in, d_count, out, status);
+    soa_to_aos_kernel<<<evolve_grid(in.cap, 152), 256, 0, s>>>(in, d_count, d_total, hit, out, hit_out, status);
     ++g_launches;
     return cudaGetLastError();
 }

@@ -15,6 +15,7 @@
 //   per-thread stack; boxes are padded so every triangle whose test can
 //   succeed is visited, and the same lexicographic rule makes the result
 //   identical to brute force.
+#include <algorithm>
 #include <cstdio>
 #include <mutex>
 #include <unordered_map>

@@ -204,8 +204,18 @@ struct GenParams {
 };
 cudaError_t launch_generate_soa(const GenParams& g, int64_t n, RaySoA out, int64_t* d_count, cudaStream_t s);
 cudaError_t launch_generate_aos(const GenParams& g, int64_t n, splat_adray_t* out, cudaStream_t s);
-cudaError_t launch_aos_to_soa(const splat_adray_t* in, int64_t n, RaySoA out, int64_t* d_count, cudaStream_t s);
-cudaError_t launch_soa_to_aos(RaySoA in, const int64_t* d_count, splat_adray_t* out, int status, cudaStream_t s);
+// active rays to out (their number added to d_count), the others to idle
+// (d_idle); ids are the rays' slots
+cudaError_t launch_aos_to_soa(const splat_adray_t* in, int64_t n, RaySoA out, int64_t* d_count, RaySoA idle,
+                              int64_t* d_idle, cudaStream_t s);
+// *d_total = *d_count + *d_idle, with the idle rays' hit state (position,
+// direction, ignored triangle, id) appended to rays [0, *d_count)
+cudaError_t launch_append_idle(RaySoA rays, const int64_t* d_count, RaySoA idle, const int64_t* d_idle,
+                               int64_t* d_total, int sm_count, cudaStream_t s);
+// rays [0, *d_count) back to their records, and the hits of [0, *d_total) to
+// their slots
+cudaError_t launch_soa_to_aos(RaySoA in, const int64_t* d_count, const int64_t* d_total, const int32_t* hit,
+                              splat_adray_t* out, int32_t* hit_out, int status, cudaStream_t s);
 
 // evolve (+ compaction, + fused splat in trace mode)
 struct SplatParams {
@@ -239,6 +249,7 @@ struct EvolveArgs {
     int32_t quirks;
     int32_t last;           // trace mode: last bounce, no optics
     splat_adray_t* aos;     // plugin mode: retired rays written back here
+    int32_t* aos_hit;       // plugin mode: and the hit they retired with, by slot
     RaySoA splat_q;         // trace mode: final-evolved diffuse rays (ignore = hit triangle)
     int64_t* splat_count;
     RaySoA sky_q;           // camera mode: rays that escaped, unchanged
