@@ -488,7 +488,7 @@ splat_status_t splat_server_status(const splat_server_t* server, int32_t* queued
  * maps: summation order only); the autotuner (splat_gb300/autotune.py)
  * picks them per workload. */
 enum {
-    SPLAT_TUNE_BRUTE_BLOCKS_PER_SM = 0, /* brute force: triangle-range splits target (default 4) */
+    SPLAT_TUNE_BRUTE_BLOCKS_PER_SM = 0, /* brute force: triangle-range splits target, in 1024 threads (default 4) */
     SPLAT_TUNE_BVH_BLOCKS_PER_SM = 1,   /* BVH traversal grid (default 16) */
     SPLAT_TUNE_EVOLVE_BLOCKS_PER_SM = 2, /* evolve grid (default 8) */
     SPLAT_TUNE_SPLAT_BLOCKS_PER_SM = 3,  /* splat grid (default 8) */
@@ -504,8 +504,8 @@ enum {
     SPLAT_TUNE_TRACE_SPLIT = 8,          /* fused trace step: the rays as 1..4 independent ranges traced on
                                             concurrent streams (steps of at least 2^17 rays; default 2) */
     SPLAT_TUNE_TEST_WAIT_STALL = 9,      /* test only (default 0, off): k > 0 makes the brute-force hitter's wait for
-                                            tile k - 1 of every block poll a barrier that nothing completes (64
-                                            polls), so each block takes the failure path of its bounded waits:
+                                            tile k - 1 of every block that needs it poll a barrier that nothing completes
+                                            (64 polls), so each such block takes the failure path of its bounded waits:
                                             error bit 1, bounded drain of its copies in flight, early return */
     SPLAT_TUNE_RAY_ORDER = 10,           /* fused trace step, four-wide BVH: 0 secondary rays traced in compaction
                                             order; 4..22 each bounce after the first groups its rays by (direction

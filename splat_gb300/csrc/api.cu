@@ -165,14 +165,13 @@ struct splat_scene {
     int device = 0;
     int64_t n_tris = 0, first_diffuse = 0;
     splat_ftri_t* d_ftri = nullptr;
-    TriHit* d_brute = nullptr;
-    TriBox* d_boxes = nullptr;   // padded boxes of the brute-force records
+    TriHit* d_recs = nullptr;    // hit records in the order of d_order
+    TriBox* d_boxes = nullptr;   // their padded boxes (BruteBoxes)
     unsigned* d_scale = nullptr; // max |vertex coordinate| (float bits), sets the box padding
     int64_t n_recs = 0;
     BvhNode* d_nodes = nullptr;
     int64_t n_nodes = 0;
-    TriHit* d_bvh = nullptr;
-    int32_t* d_order = nullptr;
+    int32_t* d_order = nullptr;  // reference index of each record: the BVH's leaf order, or a spatial one
     int32_t* d_bvh_pos = nullptr;  // inverse of d_order (n_tris + 1 entries, by reference index)
     int32_t* d_links = nullptr;  // refit links of the two-child tree
     Bvh4Node* d_nodes4 = nullptr;
@@ -196,11 +195,10 @@ struct splat_scene {
 static void scene_free(splat_scene* s) {
     if (!s) return;
     cudaFree(s->d_ftri);
-    cudaFree(s->d_brute);
+    cudaFree(s->d_recs);
     cudaFree(s->d_boxes);
     cudaFree(s->d_scale);
     cudaFree(s->d_nodes);
-    cudaFree(s->d_bvh);
     cudaFree(s->d_order);
     cudaFree(s->d_bvh_pos);
     cudaFree(s->d_links);
@@ -220,16 +218,16 @@ static cudaError_t dalloc(T** p, size_t bytes, int64_t& total) {
 
 static splat_status_t scene_pack(splat_scene* s, cudaStream_t st) {
     ProfScope ps(SPLAT_KERNEL_AUX, st);
-    cudaError_t e = launch_pack_hits(s->d_ftri, s->n_tris, s->d_brute, s->d_boxes, s->d_scale, s->d_order, s->d_bvh,
-                                     s->d_bvh_pos, st);
+    cudaError_t e = launch_pack_hits(s->d_ftri, s->n_tris, s->d_recs, s->d_boxes, s->d_scale, s->d_order, s->d_bvh_pos,
+                                     st);
     if (e != cudaSuccess) return cuda_fail(e, "pack hit records");
     if (s->d_nodes && s->d_links) {
-        e = launch_refit_tree(s->d_nodes, false, s->d_nodes4, s->n_nodes, s->d_links, s->d_flags, s->d_bvh, s->d_ftri, s->d_scale,
+        e = launch_refit_tree(s->d_nodes, false, s->d_nodes4, s->n_nodes, s->d_links, s->d_flags, s->d_recs, s->d_ftri, s->d_scale,
                               s->pad_rel, st);
         if (e != cudaSuccess) return cuda_fail(e, "BVH refit");
     }
     if (s->d_nodes4 && s->d_links4) {
-        e = launch_refit_tree(s->d_nodes4, true, s->d_nodes4, s->n_nodes4, s->d_links4, s->d_flags, s->d_bvh, s->d_ftri, s->d_scale,
+        e = launch_refit_tree(s->d_nodes4, true, s->d_nodes4, s->n_nodes4, s->d_links4, s->d_flags, s->d_recs, s->d_ftri, s->d_scale,
                               s->pad_rel, st);
         if (e != cudaSuccess) return cuda_fail(e, "BVH4 refit");
     }
@@ -290,21 +288,22 @@ splat_status_t splat_scene_create(const splat_ftri_t* host_tris, int64_t n_tris,
             delete s;
             return fail(SPLAT_ERR_INVALID, "scene_create: " + err);
         }
+    } else {
+        spatial_order(host_tris, n_tris, bvh.order);
     }
     cudaError_t e = cudaSuccess;
     auto chk = [&](cudaError_t x) {
         if (e == cudaSuccess && x != cudaSuccess) e = x;
     };
     chk(dalloc(&s->d_ftri, sizeof(splat_ftri_t) * (size_t)n_tris, s->bytes));
-    chk(dalloc(&s->d_brute, sizeof(TriHit) * (size_t)s->n_recs, s->bytes));
-    chk(dalloc(&s->d_boxes, sizeof(TriBox) * (size_t)s->n_recs, s->bytes));
+    chk(dalloc(&s->d_recs, sizeof(TriHit) * (size_t)s->n_recs, s->bytes));
+    chk(dalloc(&s->d_order, sizeof(int32_t) * (size_t)s->n_recs, s->bytes));
+    chk(dalloc(&s->d_boxes, sizeof(TriBox) * (size_t)brute_box_count(s->n_recs), s->bytes));
     chk(dalloc(&s->d_scale, sizeof(unsigned), s->bytes));
     chk(dalloc(&s->d_err, sizeof(int32_t) * 4, s->bytes));
     if (build_bvh_flag && !bvh.nodes.empty()) {
         s->n_nodes = (int64_t)bvh.nodes.size();
         chk(dalloc(&s->d_nodes, sizeof(BvhNode) * bvh.nodes.size(), s->bytes));
-        chk(dalloc(&s->d_bvh, sizeof(TriHit) * (size_t)s->n_recs, s->bytes));
-        chk(dalloc(&s->d_order, sizeof(int32_t) * bvh.order.size(), s->bytes));
         chk(dalloc(&s->d_bvh_pos, sizeof(int32_t) * ((size_t)n_tris + 1), s->bytes));
         chk(dalloc(&s->d_links, sizeof(int32_t) * bvh.links.size(), s->bytes));
         s->n_nodes4 = (int64_t)bvh.nodes4.size();
@@ -325,10 +324,9 @@ splat_status_t splat_scene_create(const splat_ftri_t* host_tris, int64_t n_tris,
     }
     chk(cudaMemcpyAsync(s->d_ftri, host_tris, sizeof(splat_ftri_t) * (size_t)n_tris, cudaMemcpyHostToDevice, st));
     chk(cudaMemsetAsync(s->d_err, 0, sizeof(int32_t) * 4, st));
+    chk(cudaMemcpyAsync(s->d_order, bvh.order.data(), sizeof(int32_t) * bvh.order.size(), cudaMemcpyHostToDevice, st));
     if (s->d_nodes) {
         chk(cudaMemcpyAsync(s->d_nodes, bvh.nodes.data(), sizeof(BvhNode) * bvh.nodes.size(), cudaMemcpyHostToDevice,
-                            st));
-        chk(cudaMemcpyAsync(s->d_order, bvh.order.data(), sizeof(int32_t) * bvh.order.size(), cudaMemcpyHostToDevice,
                             st));
         chk(cudaMemcpyAsync(s->d_links, bvh.links.data(), sizeof(int32_t) * bvh.links.size(), cudaMemcpyHostToDevice,
                             st));
@@ -338,8 +336,7 @@ splat_status_t splat_scene_create(const splat_ftri_t* host_tris, int64_t n_tris,
                             cudaMemcpyHostToDevice, st));
     }
     if (e == cudaSuccess)
-        chk(launch_pack_hits(s->d_ftri, n_tris, s->d_brute, s->d_boxes, s->d_scale, s->d_order, s->d_bvh,
-                             s->d_bvh_pos, st));
+        chk(launch_pack_hits(s->d_ftri, n_tris, s->d_recs, s->d_boxes, s->d_scale, s->d_order, s->d_bvh_pos, st));
     // host vectors above must outlive the async copies
     if (e == cudaSuccess) chk(cudaStreamSynchronize(st));
     if (e != cudaSuccess) {
@@ -406,14 +403,6 @@ static splat_status_t scene_rebuild_gpu(splat_scene* s, cudaStream_t st) {
     };
     SPLAT_CUDA(grow(&s->d_nodes, s->cap_nodes, need, sizeof(BvhNode)), "scene_rebuild: node array");
     SPLAT_CUDA(grow(&s->d_nodes4, s->cap_nodes4, need, sizeof(Bvh4Node)), "scene_rebuild: four-wide node array");
-    if (!s->d_bvh) {
-        int64_t cap = 0;
-        SPLAT_CUDA(grow(&s->d_bvh, cap, np, sizeof(TriHit)), "scene_rebuild: hit records");
-    }
-    if (!s->d_order) {
-        int64_t cap = 0;
-        SPLAT_CUDA(grow(&s->d_order, cap, np, sizeof(int32_t)), "scene_rebuild: order");
-    }
     if (!s->d_bvh_pos) {
         int64_t cap = 0;
         SPLAT_CUDA(grow(&s->d_bvh_pos, cap, s->n_tris + 1, sizeof(int32_t)), "scene_rebuild: order inverse");
@@ -426,8 +415,7 @@ static splat_status_t scene_rebuild_gpu(splat_scene* s, cudaStream_t st) {
     SPLAT_CUDA(launch_lbvh_build(s->d_ftri, s->n_tris, kLbvhLeaf, s->d_lbvh, s->d_nodes, s->d_nodes4, s->d_order,
                                  sm_count_current(), st),
                "scene_rebuild: build");
-    SPLAT_CUDA(launch_pack_hits(s->d_ftri, s->n_tris, s->d_brute, s->d_boxes, s->d_scale, s->d_order, s->d_bvh,
-                                s->d_bvh_pos, st),
+    SPLAT_CUDA(launch_pack_hits(s->d_ftri, s->n_tris, s->d_recs, s->d_boxes, s->d_scale, s->d_order, s->d_bvh_pos, st),
                "scene_rebuild: pack");
     s->gpu_bvh = true;
     s->n_nodes = need;
@@ -523,17 +511,17 @@ static splat_status_t hit_any(const splat_scene_t* s, int32_t hitter, const RayS
     if (bvh) {
         if (!s->d_nodes) {
             if (s->n_recs > 0) return fail(SPLAT_ERR_INVALID, "BVH hitter on a scene created without BVH");
-            e = launch_hit_brute(src, cap, s->d_brute, s->d_boxes, 0, hit_idx, hit_t, nullptr, s->d_err,
+            e = launch_hit_brute(src, cap, s->d_recs, s->d_boxes, 0, hit_idx, hit_t, nullptr, s->d_err,
                                  sm_count_current(), st);
         } else if (hitter == SPLAT_HITTER_BVH) {
-            e = launch_hit_bvh4(src, cap, Bvh4View{s->d_nodes4, s->d_bvh}, hit_idx, hit_t, s->d_err,
+            e = launch_hit_bvh4(src, cap, Bvh4View{s->d_nodes4, s->d_recs}, hit_idx, hit_t, s->d_err,
                                 sm_count_current(), st);
         } else {
-            e = launch_hit_bvh(src, cap, BvhView{s->d_nodes, s->d_bvh, s->d_nodes4}, hit_idx, hit_t, s->d_err, sm_count_current(),
+            e = launch_hit_bvh(src, cap, BvhView{s->d_nodes, s->d_recs, s->d_nodes4}, hit_idx, hit_t, s->d_err, sm_count_current(),
                                st);
         }
     } else if (hitter == SPLAT_HITTER_BRUTE) {
-        e = launch_hit_brute(src, cap, s->d_brute, s->d_boxes, s->n_recs, hit_idx, hit_t, tmp, s->d_err,
+        e = launch_hit_brute(src, cap, s->d_recs, s->d_boxes, s->n_recs, hit_idx, hit_t, tmp, s->d_err,
                              sm_count_current(), st);
     } else {
         return fail(SPLAT_ERR_INVALID, "unknown hitter");
@@ -1500,7 +1488,7 @@ splat_status_t splat_batch_admit(splat_batch_t* b, const splat_scene_t* scene, c
     g.seed = P->seed;
     g.light_index = 0;
     g.ray_begin = rb;
-    BatchSceneRef sc{scene->d_ftri, scene->d_brute, scene->d_boxes, scene->d_nodes4, scene->d_bvh, scene->n_recs,
+    BatchSceneRef sc{scene->d_ftri, scene->d_recs, scene->d_boxes, scene->d_nodes4, scene->d_recs, scene->n_recs,
                      scene->n_tris, scene->first_diffuse, scene->d_bvh_pos};
     const SplatParams sp =
         make_splat(P->spectrum, P->n_lambda, P->upscale, d_map, P->accum, P->frac_bits, P->map_w, P->map_h);

@@ -290,6 +290,55 @@ void prim_box(const splat_ftri_t& t, const BvhFrame& f, float pad_abs, float pad
     }
 }
 
+void spatial_order(const splat_ftri_t* tris, int64_t n_tris, std::vector<int32_t>& order) {
+    const int64_t np = n_tris - 1;
+    order.resize((size_t)std::max<int64_t>(np, 0));
+    if (np <= 0) return;
+    float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
+    std::vector<float> c((size_t)(3 * np));
+    for (int64_t j = 0; j < np; ++j) {
+        const splat_ftri_t& t = tris[j + 1];
+        for (int a = 0; a < 3; ++a) {
+            const float x = t.v[1][a], y = t.v[2][a], z = t.v[3][a];
+            const float m = 0.5f * (std::min(std::min(x, y), z) + std::max(std::max(x, y), z));
+            const float v = std::isfinite(m) ? m : 0.0f;
+            lo[a] = std::min(lo[a], v);
+            hi[a] = std::max(hi[a], v);
+            c[(size_t)(3 * j + a)] = v;
+        }
+    }
+    float scale[3];
+    for (int a = 0; a < 3; ++a) scale[a] = hi[a] > lo[a] ? 1024.0f / (hi[a] - lo[a]) : 0.0f;
+    auto spread = [](uint32_t x) {
+        x = (x | (x << 16)) & 0x030000ffu;
+        x = (x | (x << 8)) & 0x0300f00fu;
+        x = (x | (x << 4)) & 0x030c30c3u;
+        return (x | (x << 2)) & 0x09249249u;
+    };
+    // codes of 30 bits, sorted by three counting passes of 10
+    std::vector<uint64_t> key((size_t)np), tmp((size_t)np);
+    for (int64_t j = 0; j < np; ++j) {
+        uint32_t code = 0;
+        for (int a = 0; a < 3; ++a) {
+            const float f = (c[(size_t)(3 * j + a)] - lo[a]) * scale[a];
+            code |= spread(f > 0.0f ? (uint32_t)std::min(f, 1023.0f) : 0u) << a;
+        }
+        key[(size_t)j] = (uint64_t)code << 32 | (uint64_t)(j + 2);
+    }
+    for (int shift = 32; shift < 62; shift += 10) {
+        size_t at[1024] = {0}, sum = 0;
+        for (const uint64_t k : key) ++at[(k >> shift) & 1023];
+        for (size_t& n : at) {
+            const size_t m = n;
+            n = sum;
+            sum += m;
+        }
+        for (const uint64_t k : key) tmp[at[(k >> shift) & 1023]++] = k;
+        key.swap(tmp);
+    }
+    for (int64_t j = 0; j < np; ++j) order[(size_t)j] = (int32_t)(uint32_t)key[(size_t)j];
+}
+
 bool build_bvh(const splat_ftri_t* tris, int64_t n_tris, BvhHost& out, std::string& err) {
     out = BvhHost();
     const int64_t np = n_tris - 1;  // the sentinel (index 1) is never hit

@@ -22,6 +22,10 @@ struct BvhHost {
     int depth4 = 0;
 };
 
+// Reference indices 2 .. n_tris along a Morton curve of their centroids (10
+// bits an axis), for scenes without a BVH.
+void spatial_order(const splat_ftri_t* tris, int64_t n_tris, std::vector<int32_t>& order);
+
 bool build_bvh(const splat_ftri_t* tris, int64_t n_tris, BvhHost& out, std::string& err);
 // Padded box of a triangle in a frame.
 void prim_box(const splat_ftri_t& t, const BvhFrame& f, float pad_abs, float pad_rel, float lo[3], float hi[3]);

@@ -79,24 +79,6 @@ __device__ __forceinline__ float tri_t_from(float num, float den, const float4& 
     return t;
 }
 
-// The reference's test on one hoisted record (src/geo.jl:433-466).
-__device__ __forceinline__ float tri_t(const float4& q0, const float4& q1, const float4& q2, const float4& q3,
-                                       const float4& q4, const HitRay& r, bool& inside) {
-    float num = q0.w - ((q0.x * r.ox + q0.y * r.oy) + q0.z * r.oz);
-    float den = (q0.x * r.dx + q0.y * r.dy) + q0.z * r.dz;
-    float t = num / den;
-    float px = r.ox + r.dx * t;
-    float py = r.oy + r.dy * t;
-    float pz = r.oz + r.dz * t;
-    float v2x = px - q1.x, v2y = py - q1.y, v2z = pz - q1.z;
-    float d02 = (q2.x * v2x + q2.y * v2y) + q2.z * v2z;
-    float d12 = (q3.x * v2x + q3.y * v2y) + q3.z * v2z;
-    float u = (q3.w * d02 - q4.x * d12) * q4.y;
-    float v = (q2.w * d12 - q4.x * d02) * q4.y;
-    inside = (u >= 0.0f) & (v >= 0.0f) & (u + v < 1.0f);
-    return t;
-}
-
 __device__ __forceinline__ float safe_inv(float d) {
     return 1.0f / (fabsf(d) > 1.0e-30f ? d : copysignf(1.0e-30f, d));
 }
@@ -692,9 +674,9 @@ __device__ __forceinline__ bool packet_coherent(const HitRay& r, int form, float
     return ds <= dir_spread && os <= org_spread * extent;
 }
 
-// Closest hit of one ray over hit records in reference-index order (the
-// per-ray form of the brute-force hitter; strict < keeps the smaller index),
-// each record behind its padded box as in the tiled kernel.
+// Closest hit of one ray over hit records in any order (the per-ray form of
+// the brute-force hitter; ties take the smaller index), each record behind
+// its padded box as in the tiled kernel.
 __device__ __forceinline__ void brute_closest(const HitRay& r, const TriHit* recs, const TriBox* boxes,
                                               int64_t n_recs, float& best_out, int32_t& bi_out) {
     float best = __int_as_float(0x7f800000);
@@ -716,7 +698,7 @@ __device__ __forceinline__ void brute_closest(const HitRay& r, const TriHit* rec
         const int32_t idx = __float_as_int(q1.w);
         bool inside;
         const float t = tri_t_from(num, den, q1, __ldg(&h->e0), __ldg(&h->e1), __ldg(&h->inv), r, inside);
-        if (inside & (t > 0.0f) & (idx != r.ig) & (t < best)) {
+        if (inside & (t > 0.0f) & (idx != r.ig) & ((t < best) | ((t == best) & (idx < bi)))) {
             best = t;
             bi = idx;
         }

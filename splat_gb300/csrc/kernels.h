@@ -129,8 +129,20 @@ struct BvhView {
     const Bvh4Node* root4;  // the four-wide tree over the same leaves: its root holds the frame
 };
 
-// brute force over prepacked hit records (reference indices 2..T in order),
-// each behind its padded box
+// The padded boxes of the brute-force records in one array: one per record,
+// then one per 8 and one per 32 consecutive records.
+struct BruteBoxes {
+    const TriBox *box, *box8, *box32;
+};
+__host__ __device__ inline int64_t brute_box_count(int64_t n_recs) {
+    return n_recs + (n_recs + 7) / 8 + (n_recs + 31) / 32;
+}
+__host__ __device__ inline BruteBoxes brute_boxes_of(const TriBox* all, int64_t n_recs) {
+    return {all, all + n_recs, all + n_recs + (n_recs + 7) / 8};
+}
+
+// brute force over prepacked hit records (reference indices 2..T in any
+// order), each behind its padded box
 cudaError_t launch_hit_brute(const RaySrc& rays, int64_t cap, const TriHit* recs, const TriBox* boxes, int64_t n_recs,
                              int32_t* hit_idx, float* hit_t, uint64_t* tmp, int32_t* err, int sm_count,
                              cudaStream_t s);
@@ -187,10 +199,10 @@ cudaError_t launch_order_scan(uint32_t* cnt, int64_t buckets, uint32_t* sums, cu
 
 // scene packing / refit.  scale: device word holding max |vertex coordinate|
 // (float bits), from which every padded box takes pad_abs = 1e-4 max(1, scale).
-// bvh_pos (optional, n_tris + 1 entries): the inverse of bvh_order.
-cudaError_t launch_pack_hits(const splat_ftri_t* ftri, int64_t n_tris, TriHit* brute_recs, TriBox* brute_boxes,
-                             unsigned* scale, const int32_t* bvh_order, TriHit* bvh_recs, int32_t* bvh_pos,
-                             cudaStream_t s);
+// order: reference index of each record; bvh_pos (optional, n_tris + 1
+// entries): its inverse.
+cudaError_t launch_pack_hits(const splat_ftri_t* ftri, int64_t n_tris, TriHit* recs, TriBox* boxes, unsigned* scale,
+                             const int32_t* order, int32_t* bvh_pos, cudaStream_t s);
 
 
 // generation and conversion
