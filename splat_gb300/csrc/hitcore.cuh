@@ -120,6 +120,18 @@ __device__ __forceinline__ float min3f(float a, float b, float c) {
     return d;
 }
 
+// Two binary32 fused multiply-adds in one instruction (sm_100 and later),
+// each rounded as fmaf rounds it.
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+    float2 d;
+    asm("{\n\t.reg .b64 x, y, z, w;\n\t"
+        "mov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tmov.b64 z, {%6, %7};\n\t"
+        "fma.rn.f32x2 w, x, y, z;\n\tmov.b64 {%0, %1}, w;\n\t}"
+        : "=f"(d.x), "=f"(d.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+    return d;
+}
+
 // Entry and exit distances of a ray through the four child boxes of a
 // node.  The slab planes are picked by the signs of the inverse direction
 // (ix < 0: the near x plane is hi, else lo), through the addresses of the
@@ -138,11 +150,20 @@ __device__ __forceinline__ void node4_slabs(const Bvh4Node* nd, float ix, float 
     const float4 nx = __ldg(q + sx), fx = __ldg(q + 1 - sx);
     const float4 ny = __ldg(q + 2 + sy), fy = __ldg(q + 3 - sy);
     const float4 nz = __ldg(q + 4 + sz), fz = __ldg(q + 5 - sz);
+    const float2 ix2 = make_float2(ix, ix), iy2 = make_float2(iy, iy), iz2 = make_float2(iz, iz);
+    const float2 ox2 = make_float2(-oix, -oix), oy2 = make_float2(-oiy, -oiy), oz2 = make_float2(-oiz, -oiz);
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        t0[i] = max3f(fmaf(comp(nx, i), ix, -oix), fmaf(comp(ny, i), iy, -oiy),
-                      fmaxf(fmaf(comp(nz, i), iz, -oiz), 0.0f));
-        tmax[i] = min3f(fmaf(comp(fx, i), ix, -oix), fmaf(comp(fy, i), iy, -oiy), fmaf(comp(fz, i), iz, -oiz));
+    for (int i = 0; i < 4; i += 2) {
+        const float2 ax = fma2(make_float2(comp(nx, i), comp(nx, i + 1)), ix2, ox2);
+        const float2 ay = fma2(make_float2(comp(ny, i), comp(ny, i + 1)), iy2, oy2);
+        const float2 az = fma2(make_float2(comp(nz, i), comp(nz, i + 1)), iz2, oz2);
+        const float2 bx = fma2(make_float2(comp(fx, i), comp(fx, i + 1)), ix2, ox2);
+        const float2 by = fma2(make_float2(comp(fy, i), comp(fy, i + 1)), iy2, oy2);
+        const float2 bz = fma2(make_float2(comp(fz, i), comp(fz, i + 1)), iz2, oz2);
+        t0[i] = max3f(ax.x, ay.x, fmaxf(az.x, 0.0f));
+        t0[i + 1] = max3f(ax.y, ay.y, fmaxf(az.y, 0.0f));
+        tmax[i] = min3f(bx.x, by.x, bz.x);
+        tmax[i + 1] = min3f(bx.y, by.y, bz.y);
     }
 }
 
