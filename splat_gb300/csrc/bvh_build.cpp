@@ -172,7 +172,7 @@ struct Builder {
 // spanned by a sampled triangle's normal and one of its edges, and a frame is
 // judged by the sum of sqrt(half box area) over a sample of triangles, i.e.
 // by box size weighted neither to the few largest triangles (a room's walls)
-// nor to the many smallest.  The sample is a fixed stride, so a build is
+// nor to the many smallest.  The sample is a fixed one, so a build is
 // reproducible.
 //
 // kFrameGain: the world frame stays unless a candidate's sum is below this
@@ -186,8 +186,8 @@ struct Builder {
 // candidate wins by sampling noise alone (shares above 0.97) and turning the
 // rays costs 3 % (sphere 1.16 -> 1.20 ms, displaced sphere 1.35 -> 1.40 ms
 // when any smaller sum is taken), hence a line below that noise.
-constexpr int kFrameTris = 24;    // triangles that propose frames, three each
-constexpr int kFrameSample = 384; // triangles that judge them
+constexpr int kFrameTris = 8;     // triangles that propose frames, three each
+constexpr int kFrameSample = 256; // triangles that judge them
 constexpr float kFrameGain = 0.96f;
 
 struct Quat {
@@ -217,12 +217,20 @@ Quat quat_of_rows(const double e[3][3]) {
     return {(float)(sg * q[0]), (float)(sg * q[1]), (float)(sg * q[2])};
 }
 
-double frame_cost(const splat_ftri_t* tris, int64_t np, int64_t stride, const BvhFrame& f, float pad_abs,
-                  float pad_rel) {
+// The k-th of m triangles picked out of np: spread by the golden ratio, which
+// falls in step with no mesh generator's period.
+int64_t picked(int64_t k, int64_t m, int64_t np) {
+    if (m >= np) return k;
+    const uint64_t frac = (uint64_t)k * 0x9E3779B97F4A7C15ull >> 32;
+    return (int64_t)(frac * (uint64_t)np >> 32);
+}
+
+double frame_cost(const splat_ftri_t* tris, int64_t np, const BvhFrame& f, float pad_abs, float pad_rel) {
     double sum = 0.0;
-    for (int64_t j = 0; j < np; j += stride) {
+    const int64_t m = std::min<int64_t>(np, kFrameSample);
+    for (int64_t k = 0; k < m; ++k) {
         float lo[3], hi[3];
-        prim_box(tris[j + 1], f, pad_abs, pad_rel, lo, hi);
+        prim_box(tris[picked(k, m, np) + 1], f, pad_abs, pad_rel, lo, hi);
         const double x = hi[0] - lo[0], y = hi[1] - lo[1], z = hi[2] - lo[2];
         const double a = x * y + y * z + z * x;
         if (std::isfinite(a)) sum += std::sqrt(a);
@@ -232,13 +240,12 @@ double frame_cost(const splat_ftri_t* tris, int64_t np, int64_t stride, const Bv
 
 Quat pick_frame(const splat_ftri_t* tris, int64_t np, float pad_abs, float pad_rel) {
     const Quat world{0.0f, 0.0f, 0.0f};
-    const int64_t stride = np > kFrameSample ? np / kFrameSample : 1;
-    const double base = frame_cost(tris, np, stride, frame_of(0.0f, 0.0f, 0.0f), pad_abs, pad_rel);
+    const double base = frame_cost(tris, np, frame_of(0.0f, 0.0f, 0.0f), pad_abs, pad_rel);
     Quat best = world;
     double best_cost = kFrameGain * base;
-    const int64_t from = np > kFrameTris ? np / kFrameTris : 1;
-    for (int64_t j = 0; j < np; j += from) {
-        const splat_ftri_t& t = tris[j + 1];
+    const int64_t proposers = std::min<int64_t>(np, kFrameTris);
+    for (int64_t k = 0; k < proposers; ++k) {
+        const splat_ftri_t& t = tris[picked(k, proposers, np) + 1];
         for (int edge = 0; edge < 3; ++edge) {
             const float* p = t.v[1 + edge];
             const float* q = t.v[1 + (edge + 1) % 3];
@@ -260,7 +267,7 @@ Quat pick_frame(const splat_ftri_t* tris, int64_t np, float pad_abs, float pad_r
                 e[1][k] = e[2][(k + 1) % 3] * e[0][(k + 2) % 3] - e[2][(k + 2) % 3] * e[0][(k + 1) % 3];
             const Quat c = quat_of_rows(e);
             if (!std::isfinite(c.x) || !std::isfinite(c.y) || !std::isfinite(c.z)) continue;
-            const double cost = frame_cost(tris, np, stride, frame_of(c.x, c.y, c.z), pad_abs, pad_rel);
+            const double cost = frame_cost(tris, np, frame_of(c.x, c.y, c.z), pad_abs, pad_rel);
             if (cost < best_cost) {
                 best_cost = cost;
                 best = c;
