@@ -868,6 +868,9 @@ static splat_status_t trace_part(const splat_scene_t* scene, const splat_trace_p
             // same order, so its survivors leave as compact patches
             const int64_t gh = P->light.res1 / P->upscale;
             if (b == 1 && rb % gh == 0 && gh <= (int64_t)kGridTileMaxRows) src.tile_h = (int32_t)gh;
+            if (b == 1 && src.packet == 1 && g_tune[SPLAT_TUNE_BVH_PACKET] == 1 &&
+                !packet_density(grid_rays(P), scene->n_recs))
+                src.packet = 0;
         }
         if (b >= 2 && order_bits > 0 && P->hitter == SPLAT_HITTER_BVH && scene->d_nodes4 && scene->d_bvh_pos) {
             // secondary rays in coherent order: (octant, position of the triangle they leave)
@@ -2022,6 +2025,8 @@ splat_status_t splat_render_camera_after(const splat_scene_t* scene, const splat
         // camera rays are the sub-sample grid's columns in order: first-bounce
         // packets take 8 x 4 tiles of it
         if (b == 1 && ch <= (int64_t)kGridTileMaxRows) src.tile_h = (int32_t)ch;
+        if (b == 1 && src.packet == 1 && g_tune[SPLAT_TUNE_BVH_PACKET] == 1 && !packet_density(cnt, scene->n_recs))
+            src.packet = 0;
         rc = hit_any(scene, P->hitter, src, cnt, w.hit, nullptr, w.tmp, st);
         if (rc != SPLAT_OK) return rc;
         ea.in = cur;

@@ -53,7 +53,7 @@ struct BatchItem {
     int32_t start_tick;  // tick of the first bounce; < 0: slot unused
     int32_t quirks;
     float force_rand;
-    int32_t _pad0;
+    int32_t dense;       // enough rays for its triangles that first-bounce packets pay (packet_density)
     GenParams gen;
     int64_t n_rays;
     splat_material_t material;
@@ -214,7 +214,8 @@ __device__ __forceinline__ void hit_phase(RaySoA in, const int64_t* __restrict__
         const uint32_t slot0 = __shfl_sync(0xffffffffu, slot, 0);
         bool packet = false;
         if (packet_mode > 0 && __all_sync(0xffffffffu, bvh & (slot == slot0))) {
-            const int form = packet_form(packet_mode, tick == it.start_tick);  // warp-uniform: one item
+            // warp-uniform: one item
+            const int form = packet_mode == 1 && !it.dense ? 0 : packet_form(packet_mode, tick == it.start_tick);
             packet = form == 1 || (form >= 2 && packet_coherent(r, form, bvh4_extent(it.nodes4)));
         }
         float best;
@@ -657,6 +658,7 @@ void batch_fill_item(void* dst, const BatchSceneRef& sc, const GenParams& gen, i
     it.sp = sp;
     it.bvh_pos = sc.nodes4 ? sc.bvh_pos : nullptr;
     const int64_t rows = gen.light.res1 / gen.upscale;
+    it.dense = packet_density(rows * (gen.light.res2 / gen.upscale), sc.n_recs) ? 1 : 0;
     it.grid_rows = (rows >= 1 && rows <= (int64_t)kGridTileMaxRows && gen.ray_begin % rows == 0) ? (int32_t)rows : 0;
     std::memcpy(dst, &it, sizeof(it));
 }

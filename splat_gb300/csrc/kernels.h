@@ -29,11 +29,24 @@ struct RaySrc {
     int32_t packet;            // four-wide BVH: packet_form of the launch (0 one ray per lane)
     const int32_t* perm;       // BVH hitters: the k-th ray traced is ray perm[k] (nullptr: ray k); results
                                // go to the ray's own index
-    int32_t tile_h;            // packet kernels, no perm: rays are a light grid of tile_h rows in column-major
-                               // order; warps take 8 x 4 tiles of it (0: in order)
+    int32_t tile_h;            // packet and brute-force kernels, no perm: rays are a light grid of tile_h rows in
+                               // column-major order; warps take 8 x 4 tiles of it (0: in order)
     int32_t few;               // the count on the device may be far below the launch's bound (later bounces):
                                // four-wide BVH launches prepare for kGroupRays rays or less
 };
+
+// First-bounce rays come from a grid, and a packet of them pays where their
+// paths through the tree overlap: with few rays for the triangles a packet's
+// 8 x 4 patch spans many leaves and its warp walks them all in turn.
+// Measured on one GB300, us a one-bounce step, one lane a ray / packets, by
+// rays per triangle:
+//   displaced sphere, 81,922   0.4 148/272   0.8 152/229   1.6 183/204   3.2 226/215   12.8 481/349
+//   displaced sphere, 20,482   1.6 116/132   3.2 122/120   6.4 136/123   12.8 174/135
+//   sponge, 96,012             0.7  68/72    1.4  84/90    2.7 112/107   10.9 270/241
+constexpr float kPacketRaysPerTri = 2.5f;
+__host__ __device__ inline bool packet_density(int64_t grid_rays, int64_t n_recs) {
+    return (float)grid_rays >= kPacketRaysPerTri * (float)n_recs;
+}
 
 // Which traversal a warp of four-wide BVH rays takes, from
 // SPLAT_TUNE_BVH_PACKET and whether the rays are on their first bounce:
