@@ -807,6 +807,25 @@ static int64_t grid_rays(const splat_trace_params_t* P) {
     return (P->light.res1 / P->upscale) * (P->light.res2 / P->upscale);
 }
 
+// Whether a step of cnt rays runs as one launch: the two default hitters under
+// the default forms (a knob that asks for a form of the separate kernels gets
+// them).  Measured on one GB300, us a step, separate launches -> one, at
+// 1,024 / 4,096 / 8,100 / 16,384 / 32,761 rays (depth 3, 4 planes, 2 x 2):
+//   sphere, 322 triangles, brute force   125/131/132/133/141 -> 60/64/73/114/193
+//   displaced sphere, 81,922, BVH        111/129/146/154/444 -> 77/84/99/149/249
+//   sponge, 96,012, BVH                  122/141/175/192/247 -> 85/98/140/210/371
+//   sphere, 20,482, brute force          144/193/232/289/320 -> 163/169/188/281/452
+// and 5,472 rays on a sponge of 4,813 by brute force, depth 6: 518 -> 631 (its
+// boxes overlap, and a group meets them in no particular order).
+static bool small_step(const splat_scene_t* scene, const splat_trace_params_t* P, int64_t cnt) {
+    return cnt <= kSmallStepRays && (P->hitter == SPLAT_HITTER_BVH || P->hitter == SPLAT_HITTER_BRUTE) &&
+           (P->hitter == SPLAT_HITTER_BVH || scene->n_recs <= kSmallStepBruteRecs) &&
+           g_tune[SPLAT_TUNE_BVH_PACKET] <= 1 &&
+           g_tune[SPLAT_TUNE_BVH_REFILL] == 0 && g_tune[SPLAT_TUNE_RAY_ORDER] == 0 &&
+           g_tune[SPLAT_TUNE_SPLAT_AGGREGATE] == 0 && g_tune[SPLAT_TUNE_COUNT_WORK] == 0 &&
+           g_tune[SPLAT_TUNE_TEST_WAIT_STALL] == 0;
+}
+
 // The forward step over rays [rb, rb + cnt) of the grid in the work area w,
 // on stream st: generate, depth x {hit, evolve (+ compaction, diffuse
 // queue)}, the splat (segments on a side stream), the statistics.  The map
@@ -826,11 +845,6 @@ static splat_status_t trace_part(const splat_scene_t* scene, const splat_trace_p
     g.seed = P->seed;
     g.light_index = 0;
     g.ray_begin = rb;
-    {
-        ProfScope ps(SPLAT_KERNEL_GENERATE, st);
-        SPLAT_CUDA(launch_generate_soa(g, cnt, w.a, &w.counts[0], st), "generate");
-    }
-
     EvolveArgs ea;
     std::memset(&ea, 0, sizeof(ea));
     ea.tris = scene->d_ftri;
@@ -843,6 +857,20 @@ static splat_status_t trace_part(const splat_scene_t* scene, const splat_trace_p
     ea.quirks = (P->flags & SPLAT_FLAG_REF_QUIRKS) ? 1 : 0;
     const SplatParams sp =
         make_splat(P->spectrum, P->n_lambda, P->upscale, d_map, P->accum, P->frac_bits, P->map_w, P->map_h);
+    if (alone && small_step(scene, P, cnt)) {
+        ProfScope ps(SPLAT_KERNEL_EVOLVE, st);
+        const bool bvh = P->hitter == SPLAT_HITTER_BVH && scene->d_nodes4;
+        SPLAT_CUDA(launch_small_step(g, cnt, bvh ? scene->d_nodes4 : nullptr, scene->d_recs, scene->d_boxes,
+                                     scene->n_recs, ea, P->depth, sp, d_stats, st),
+                   "small step");
+        return SPLAT_OK;
+    }
+    SPLAT_CUDA(cudaMemsetAsync(w.counts, 0, kCounterBytes, st), "memset counters");
+    {
+        ProfScope ps(SPLAT_KERNEL_GENERATE, st);
+        SPLAT_CUDA(launch_generate_soa(g, cnt, w.a, &w.counts[0], st), "generate");
+    }
+
     ea.splat_q = w.q;
     ea.splat_count = &w.counts[kSplatCount];
     // Splat overlap: the queue segment of bounces (seg, b] is splatted on the
@@ -957,7 +985,6 @@ splat_status_t splat_trace_forward(const splat_scene_t* scene, const splat_trace
     if (P->zero_map) SPLAT_CUDA(cudaMemsetAsync(d_map, 0, (size_t)P->map_w * P->map_h * planes * 4, st), "clear map");
     if (parts == 1) {
         Work w = carve_work(d_workspace, cnt);
-        SPLAT_CUDA(cudaMemsetAsync(w.counts, 0, kCounterBytes, st), "memset counters");
         return trace_part(scene, P, d_map, w, rb, cnt, d_stats, st, sm, cnt < kSplitMinRays);
     }
     // the ranges are independent (ray ids are grid indices); each runs on its
@@ -975,7 +1002,6 @@ splat_status_t splat_trace_forward(const splat_scene_t* scene, const splat_trace
         cudaStream_t si = i == 0 ? st : side->part[i - 1];
         if (i > 0) SPLAT_CUDA(cudaStreamWaitEvent(si, side->part_ev[0], 0), "fork ranges");
         Work w = carve_work(base + (size_t)i * region, n_i);
-        SPLAT_CUDA(cudaMemsetAsync(w.counts, 0, kCounterBytes, si), "memset counters");
         splat_status_t rc = trace_part(scene, P, d_map, w, lo, n_i, d_stats, si, sm, false);
         if (rc != SPLAT_OK) return rc;
     }

@@ -102,17 +102,6 @@ constexpr int kBruteRun = 512;
 constexpr int kScanThreads = 128;
 constexpr int kScanRPT = 1;
 
-// May a ray enter the box at or before best?
-__device__ __forceinline__ bool enters(const float4& lo, const float4& hi, const float inv[3], const float oinv[3],
-                                       float best) {
-    const float a0 = fmaf(lo.x, inv[0], -oinv[0]), b0 = fmaf(hi.x, inv[0], -oinv[0]);
-    const float a1 = fmaf(lo.y, inv[1], -oinv[1]), b1 = fmaf(hi.y, inv[1], -oinv[1]);
-    const float a2 = fmaf(lo.z, inv[2], -oinv[2]), b2 = fmaf(hi.z, inv[2], -oinv[2]);
-    const float tmin = fmaxf(fmaxf(fminf(a0, b0), fminf(a1, b1)), fminf(a2, b2));
-    const float tmax = fminf(fminf(fmaxf(a0, b0), fmaxf(a1, b1)), fmaxf(a2, b2));
-    return (tmin <= tmax) & (tmax >= 0.0f) & (tmin <= best);
-}
-
 template <int RPT, bool AOS, int TILE>
 __global__ void __launch_bounds__(kScanThreads) hit_brute_kernel(RaySrc src, const TriHit* __restrict__ recs,
                                                                   BruteBoxes boxes,

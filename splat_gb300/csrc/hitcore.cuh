@@ -515,6 +515,82 @@ static_assert(kGroupStackWarp >= 4 * kGroupStack<8>, "one warp's stacks");
 constexpr int64_t kGroupWarpRays = 4096;
 constexpr int64_t kGroupRays = 16384;
 
+// One step of every group of the warp (all 32 lanes call; a group without
+// entries, sp = 0, idles).
+template <int G>
+__device__ __forceinline__ void bvh4_group_step(const HitRay& r, const SlabRay& sr, const Bvh4View& bvh, int2* stack,
+                                                int& sp, float& best, int32_t& bi) {
+    const int lane = threadIdx.x & 31, gl = lane & (G - 1), g0 = lane & ~(G - 1);
+    const unsigned gmask = G == 32 ? 0xffffffffu : ((1u << (G & 31)) - 1u) << g0;
+    const unsigned below = (1u << lane) - 1u;
+    __syncwarp();
+    const int room = (kGroupStack<G> - kBvhStack - sp) / 3;
+    const int take = min(min(sp, G), max(room, 1));
+    const bool mine = gl < take;
+    sp -= take;
+    int ref = 0;
+    bool go = false;
+    if (mine) {
+        const int2 e = stack[sp + gl];
+        ref = e.x;
+        go = __int_as_float(e.y) <= best;
+    }
+    bool h[4] = {false, false, false, false};
+    float tmin[4] = {0.f, 0.f, 0.f, 0.f};
+    int4 c = make_int4(0, 0, 0, 0);
+    float lb = best;
+    int32_t li = bi;
+    if (go && ref >= 0) {
+        const Bvh4Node* nd = bvh.nodes + ref;
+        c = __ldg(&nd->c);
+        float tmax[4];
+        node4_slabs(nd, sr.ix, sr.iy, sr.iz, sr.oix, sr.oiy, sr.oiz, tmin, tmax);
+    #pragma unroll
+        for (int i = 0; i < 4; ++i) h[i] = (tmin[i] <= tmax[i]) & (tmin[i] <= best);
+    } else if (go) {
+        const int enc = ~ref;
+        const int first = enc >> 4;
+        const int count = (enc & 15) + 1;
+        for (int j = 0; j < count; ++j) {
+            const TriHit* t3 = bvh.tris + first + j;
+            float num, den;
+            if (!tri_candidate(__ldg(&t3->n_nv), r, lb, num, den)) continue;
+            const float4 q1 = __ldg(&t3->a_idx);
+            const int32_t idx = __float_as_int(q1.w);
+            bool inside;
+            const float t = tri_t_from(num, den, q1, __ldg(&t3->e0), __ldg(&t3->e1), __ldg(&t3->inv), r, inside);
+            if (inside & (t > 0.0f) & (idx != r.ig) & ((t < lb) | ((t == lb) & (idx < li)))) {
+                lb = t;
+                li = idx;
+            }
+        }
+    }
+    __syncwarp();  // the entries taken have been read
+    if (__any_sync(0xffffffffu, (lb < best) | (li != bi))) {
+        // the group's smallest (t, index); t >= 0, so its bits order as it
+    #pragma unroll
+        for (int o = G / 2; o; o >>= 1) {
+            const float ot = __shfl_xor_sync(0xffffffffu, lb, o);
+            const int32_t oi = __shfl_xor_sync(0xffffffffu, li, o);
+            if ((ot < lb) | ((ot == lb) & (oi < li))) {
+                lb = ot;
+                li = oi;
+            }
+        }
+        best = lb;
+        bi = li;
+    }
+    #pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const unsigned m = __ballot_sync(0xffffffffu, h[i]) & gmask;
+        if (h[i]) {
+            const int ci = i == 0 ? c.x : (i == 1 ? c.y : (i == 2 ? c.z : c.w));
+            stack[sp + __popc(m & below)] = make_int2(ci, __float_as_int(tmin[i]));
+        }
+        sp += __popc(m);
+    }
+}
+
 // load(k): ray k; view(k): the BVH it is traced in; store(k, t, index).
 // Groups take rays off the work counter, or stride statically without one.
 template <int G, class Load, class View, class Store>
@@ -523,8 +599,6 @@ __device__ __forceinline__ void bvh4_group_loop(int64_t n, unsigned long long* f
     static_assert(G == 8 || G == 32, "group size");
     const float kInf = __int_as_float(0x7f800000);
     const int lane = threadIdx.x & 31, gl = lane & (G - 1), g0 = lane & ~(G - 1);
-    const unsigned gmask = G == 32 ? 0xffffffffu : ((1u << (G & 31)) - 1u) << g0;
-    const unsigned below = (1u << lane) - 1u;
     const int64_t groups = (int64_t)gridDim.x * (blockDim.x / G);
     int64_t next = (int64_t)blockIdx.x * (blockDim.x / G) + threadIdx.x / G;
     HitRay r{};
@@ -571,73 +645,22 @@ __device__ __forceinline__ void bvh4_group_loop(int64_t n, unsigned long long* f
             if (!fetch) more = __any_sync(0xffffffffu, next < n);
         }
         if (!more && __all_sync(0xffffffffu, k < 0)) break;
-        __syncwarp();
-        const int room = (kGroupStack<G> - kBvhStack - sp) / 3;
-        const int take = min(min(sp, G), max(room, 1));
-        const bool mine = gl < take;
-        sp -= take;
-        int ref = 0;
-        bool go = false;
-        if (mine) {
-            const int2 e = stack[sp + gl];
-            ref = e.x;
-            go = __int_as_float(e.y) <= best;
-        }
-        bool h[4] = {false, false, false, false};
-        float tmin[4] = {0.f, 0.f, 0.f, 0.f};
-        int4 c = make_int4(0, 0, 0, 0);
-        float lb = best;
-        int32_t li = bi;
-        if (go && ref >= 0) {
-            const Bvh4Node* nd = bvh.nodes + ref;
-            c = __ldg(&nd->c);
-            float tmax[4];
-            node4_slabs(nd, sr.ix, sr.iy, sr.iz, sr.oix, sr.oiy, sr.oiz, tmin, tmax);
-#pragma unroll
-            for (int i = 0; i < 4; ++i) h[i] = (tmin[i] <= tmax[i]) & (tmin[i] <= best);
-        } else if (go) {
-            const int enc = ~ref;
-            const int first = enc >> 4;
-            const int count = (enc & 15) + 1;
-            for (int j = 0; j < count; ++j) {
-                const TriHit* t3 = bvh.tris + first + j;
-                float num, den;
-                if (!tri_candidate(__ldg(&t3->n_nv), r, lb, num, den)) continue;
-                const float4 q1 = __ldg(&t3->a_idx);
-                const int32_t idx = __float_as_int(q1.w);
-                bool inside;
-                const float t = tri_t_from(num, den, q1, __ldg(&t3->e0), __ldg(&t3->e1), __ldg(&t3->inv), r, inside);
-                if (inside & (t > 0.0f) & (idx != r.ig) & ((t < lb) | ((t == lb) & (idx < li)))) {
-                    lb = t;
-                    li = idx;
-                }
-            }
-        }
-        __syncwarp();  // the entries taken have been read
-        if (__any_sync(0xffffffffu, (lb < best) | (li != bi))) {
-            // the group's smallest (t, index); t >= 0, so its bits order as it
-#pragma unroll
-            for (int o = G / 2; o; o >>= 1) {
-                const float ot = __shfl_xor_sync(0xffffffffu, lb, o);
-                const int32_t oi = __shfl_xor_sync(0xffffffffu, li, o);
-                if ((ot < lb) | ((ot == lb) & (oi < li))) {
-                    lb = ot;
-                    li = oi;
-                }
-            }
-            best = lb;
-            bi = li;
-        }
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const unsigned m = __ballot_sync(0xffffffffu, h[i]) & gmask;
-            if (h[i]) {
-                const int ci = i == 0 ? c.x : (i == 1 ? c.y : (i == 2 ? c.z : c.w));
-                stack[sp + __popc(m & below)] = make_int2(ci, __float_as_int(tmin[i]));
-            }
-            sp += __popc(m);
-        }
+        bvh4_group_step<G>(r, sr, bvh, stack, sp, best, bi);
     }
+}
+
+// Closest hit of one ray a group (all 32 lanes call; live: the group has a
+// ray).  stack: the group's kGroupStack<G> entries.
+template <int G>
+__device__ __forceinline__ void bvh4_closest_group(const HitRay& r, bool live, const Bvh4View& bvh, int2* stack,
+                                                   float& best, int32_t& bi) {
+    const SlabRay sr = slab_ray(r, bvh.nodes);
+    best = __int_as_float(0x7f800000);
+    bi = 1;
+    int sp = live ? 1 : 0;
+    __syncwarp();  // the stack's previous readers are done
+    if (live && (threadIdx.x & (G - 1)) == 0) stack[0] = make_int2(0, 0);
+    while (__any_sync(0xffffffffu, sp > 0)) bvh4_group_step<G>(r, sr, bvh, stack, sp, best, bi);
 }
 
 // n <= kGroupRays rays by the group size that suits their number; stack: the
@@ -695,6 +718,17 @@ __device__ __forceinline__ bool packet_coherent(const HitRay& r, int form, float
     return ds <= dir_spread && os <= org_spread * extent;
 }
 
+// May a ray enter the box at or before best?
+__device__ __forceinline__ bool enters(const float4& lo, const float4& hi, const float inv[3], const float oinv[3],
+                                       float best) {
+    const float a0 = fmaf(lo.x, inv[0], -oinv[0]), b0 = fmaf(hi.x, inv[0], -oinv[0]);
+    const float a1 = fmaf(lo.y, inv[1], -oinv[1]), b1 = fmaf(hi.y, inv[1], -oinv[1]);
+    const float a2 = fmaf(lo.z, inv[2], -oinv[2]), b2 = fmaf(hi.z, inv[2], -oinv[2]);
+    const float tmin = fmaxf(fmaxf(fminf(a0, b0), fminf(a1, b1)), fminf(a2, b2));
+    const float tmax = fminf(fminf(fmaxf(a0, b0), fmaxf(a1, b1)), fmaxf(a2, b2));
+    return (tmin <= tmax) & (tmax >= 0.0f) & (tmin <= best);
+}
+
 // Closest hit of one ray over hit records in any order (the per-ray form of
 // the brute-force hitter; ties take the smaller index), each record behind
 // its padded box as in the tiled kernel.
@@ -722,6 +756,55 @@ __device__ __forceinline__ void brute_closest(const HitRay& r, const TriHit* rec
         if (inside & (t > 0.0f) & (idx != r.ig) & ((t < best) | ((t == best) & (idx < bi)))) {
             best = t;
             bi = idx;
+        }
+    }
+    best_out = best;
+    bi_out = bi;
+}
+
+// The same over the lanes of a group of G: each takes every G-th box of 32
+// records, and the groups' results are the smallest (t, index).  All 32
+// lanes call.
+template <int G>
+__device__ __forceinline__ void brute_closest_group(const HitRay& r, bool live, const TriHit* recs,
+                                                    const TriBox* all_boxes, int64_t n_recs, float& best_out,
+                                                    int32_t& bi_out) {
+    const BruteBoxes boxes = brute_boxes_of(all_boxes, n_recs);
+    const float inv[3] = {safe_inv(r.dx), safe_inv(r.dy), safe_inv(r.dz)};
+    const float oinv[3] = {r.ox * inv[0], r.oy * inv[1], r.oz * inv[2]};
+    float best = __int_as_float(0x7f800000);
+    int32_t bi = 1;
+    const int64_t n32 = live ? (n_recs + 31) / 32 : 0;
+    for (int64_t b = threadIdx.x & (G - 1); b < n32; b += G) {
+        if (!enters(__ldg(&boxes.box32[b].lo), __ldg(&boxes.box32[b].hi), inv, oinv, best)) continue;
+        const int64_t e8 = min(4 * b + 4, (n_recs + 7) / 8);
+        for (int64_t g = 4 * b; g < e8; ++g) {
+            if (!enters(__ldg(&boxes.box8[g].lo), __ldg(&boxes.box8[g].hi), inv, oinv, best)) continue;
+            const int64_t e = min(8 * g + 8, n_recs);
+            for (int64_t j = 8 * g; j < e; ++j) {
+                if (!enters(__ldg(&boxes.box[j].lo), __ldg(&boxes.box[j].hi), inv, oinv, best)) continue;
+                const TriHit* h = recs + j;
+                float num, den;
+                if (!tri_candidate(__ldg(&h->n_nv), r, best, num, den)) continue;
+                const float4 q1 = __ldg(&h->a_idx);
+                const int32_t idx = __float_as_int(q1.w);
+                bool inside;
+                const float t = tri_t_from(num, den, q1, __ldg(&h->e0), __ldg(&h->e1), __ldg(&h->inv), r, inside);
+                if (inside & (t > 0.0f) & (idx != r.ig) & ((t < best) | ((t == best) & (idx < bi)))) {
+                    best = t;
+                    bi = idx;
+                }
+            }
+        }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int o = G / 2; o; o >>= 1) {
+        const float ot = __shfl_xor_sync(0xffffffffu, best, o);
+        const int32_t oi = __shfl_xor_sync(0xffffffffu, bi, o);
+        if ((ot < best) | ((ot == best) & (oi < bi))) {
+            best = ot;
+            bi = oi;
         }
     }
     best_out = best;

@@ -328,6 +328,16 @@ cudaError_t launch_image_accumulate(float* out, const float* rgb, int64_t n, int
 cudaError_t launch_map_to_array(const int32_t* map, int64_t w, int64_t h, int64_t planes, float inv_scale,
                                 cudaSurfaceObject_t surf, int sm_count, cudaStream_t s);
 
+// A whole trace step of at most kSmallStepRays rays in one launch (step.cu):
+// nodes4 null is the brute-force hitter; ea gives scene, material and draws
+// (its queues are unused).  stats accumulate, as launch_stats_finish leaves
+// them.
+constexpr int64_t kSmallStepRays = 12288;
+constexpr int64_t kSmallStepBruteRecs = 1024;
+cudaError_t launch_small_step(const GenParams& gen, int64_t n, const Bvh4Node* nodes4, const TriHit* recs,
+                              const TriBox* boxes, int64_t n_recs, const EvolveArgs& ea, int32_t depth,
+                              const SplatParams& sp, splat_trace_stats_t* stats, cudaStream_t s);
+
 // light-map splat of the queued diffuse rays [*d_begin, *d_count) (d_begin
 // null: from 0)
 cudaError_t launch_splat(const RaySoA& q, const int64_t* d_begin, const int64_t* d_count, const splat_ftri_t* tris,
