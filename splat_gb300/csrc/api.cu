@@ -221,15 +221,10 @@ static splat_status_t scene_pack(splat_scene* s, cudaStream_t st) {
     cudaError_t e = launch_pack_hits(s->d_ftri, s->n_tris, s->d_recs, s->d_boxes, s->d_scale, s->d_order, s->d_bvh_pos,
                                      st);
     if (e != cudaSuccess) return cuda_fail(e, "pack hit records");
-    if (s->d_nodes && s->d_links) {
-        e = launch_refit_tree(s->d_nodes, false, s->d_nodes4, s->n_nodes, s->d_links, s->d_flags, s->d_recs, s->d_ftri, s->d_scale,
-                              s->pad_rel, st);
+    if (s->d_nodes && s->d_links && s->d_nodes4 && s->d_links4) {
+        const RefitTrees t{s->d_nodes, s->d_nodes4, s->n_nodes, s->n_nodes4, s->d_links, s->d_links4, s->d_flags};
+        e = launch_refit_trees(t, s->d_recs, s->d_ftri, s->d_scale, s->pad_rel, st);
         if (e != cudaSuccess) return cuda_fail(e, "BVH refit");
-    }
-    if (s->d_nodes4 && s->d_links4) {
-        e = launch_refit_tree(s->d_nodes4, true, s->d_nodes4, s->n_nodes4, s->d_links4, s->d_flags, s->d_recs, s->d_ftri, s->d_scale,
-                              s->pad_rel, st);
-        if (e != cudaSuccess) return cuda_fail(e, "BVH4 refit");
     }
     return SPLAT_OK;
 }

@@ -176,13 +176,18 @@ cudaError_t launch_hit_bvh4(const RaySrc& rays, int64_t cap, const Bvh4View& bvh
 cudaError_t read_hit_work(uint64_t out[4], bool reset, cudaStream_t s);
 // grid of a work-counter traversal launch (one resident wave)
 int resident_grid(const void* kernel, int64_t cap, int sm_count, int threads, int max_per_sm);
-// one-launch bottom-up refit of a two-child (wide = false) or four-wide tree;
-// links: parent per node, then number of inner children per node; root4: the
-// four-wide root, whose frame the boxes are taken in
-cudaError_t launch_refit_tree(void* nodes, bool wide, const Bvh4Node* root4, int64_t n_nodes, const int32_t* links,
-                              unsigned* flags, const TriHit* bvh_recs, const splat_ftri_t* ftri,
-                              const unsigned* scale, float pad_rel, cudaStream_t s);
-
+// one-launch bottom-up refit of the two-child and the four-wide tree.  links:
+// parent per node, then number of inner children per node; flags: n2 + n4
+// arrival counts.  The boxes are taken in the frame of the four-wide root.
+struct RefitTrees {
+    BvhNode* nodes2;
+    Bvh4Node* nodes4;
+    int64_t n2, n4;
+    const int32_t *links2, *links4;
+    unsigned* flags;
+};
+cudaError_t launch_refit_trees(const RefitTrees& t, const TriHit* recs, const splat_ftri_t* ftri,
+                               const unsigned* scale, float pad_rel, cudaStream_t s);
 
 // GPU BVH rebuild (lbvh.cu): linear BVH over Morton-sorted centroids, written
 // as two-child and four-wide nodes with leaves of at most leaf_max triangles
