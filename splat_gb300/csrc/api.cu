@@ -306,7 +306,7 @@ splat_status_t splat_scene_create(const splat_ftri_t* host_tris, int64_t n_tris,
         s->cap_nodes4 = s->n_nodes4;
         chk(dalloc(&s->d_nodes4, sizeof(Bvh4Node) * bvh.nodes4.size(), s->bytes));
         chk(dalloc(&s->d_links4, sizeof(int32_t) * bvh.links4.size(), s->bytes));
-        chk(dalloc(&s->d_flags, sizeof(unsigned) * std::max(bvh.nodes.size(), bvh.nodes4.size()), s->bytes));
+        chk(dalloc(&s->d_flags, sizeof(unsigned) * (bvh.nodes.size() + bvh.nodes4.size()), s->bytes));
         s->depth = bvh.depth;
         s->max_leaf = bvh.max_leaf;
         s->leaves = bvh.leaves;
@@ -407,11 +407,9 @@ static splat_status_t scene_rebuild_gpu(splat_scene* s, cudaStream_t st) {
         SPLAT_CUDA(cudaMalloc(&s->d_lbvh, b), "scene_rebuild: scratch");
         s->bytes += (int64_t)b;
     }
-    SPLAT_CUDA(launch_lbvh_build(s->d_ftri, s->n_tris, kLbvhLeaf, s->d_lbvh, s->d_nodes, s->d_nodes4, s->d_order,
-                                 sm_count_current(), st),
+    const LbvhOut out{s->d_nodes, s->d_nodes4, s->d_order, s->d_recs, s->d_boxes, s->d_bvh_pos, s->d_scale};
+    SPLAT_CUDA(launch_lbvh_build(s->d_ftri, s->n_tris, kLbvhLeaf, s->d_lbvh, out, sm_count_current(), st),
                "scene_rebuild: build");
-    SPLAT_CUDA(launch_pack_hits(s->d_ftri, s->n_tris, s->d_recs, s->d_boxes, s->d_scale, s->d_order, s->d_bvh_pos, st),
-               "scene_rebuild: pack");
     s->gpu_bvh = true;
     s->n_nodes = need;
     s->n_nodes4 = need;

@@ -425,19 +425,6 @@ cudaError_t launch_hit_brute(const RaySrc& rays, int64_t cap, const TriHit* recs
 // ---------------------------------------------------------------------------
 // brute force over the reference's n_tris array (next_hit_kernel6 drop-in)
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ TriHit pack_one(int32_t idx, F3 n, F3 a, F3 b, F3 c) {
-    TriHit h;
-    F3 v0 = c - a, v1 = b - a;
-    float dot00 = dot(v0, v0), dot01 = dot(v0, v1), dot11 = dot(v1, v1);
-    float invDenom = 1.0f / (dot00 * dot11 - dot01 * dot01);
-    h.n_nv = make_float4(n.x, n.y, n.z, dot(n, a));
-    h.a_idx = make_float4(a.x, a.y, a.z, __int_as_float(idx));
-    h.e0 = make_float4(v0.x, v0.y, v0.z, dot00);
-    h.e1 = make_float4(v1.x, v1.y, v1.z, dot11);
-    h.inv = make_float4(dot01, invDenom, 0.f, 0.f);
-    return h;
-}
-
 // Box of a caller's record outside which no point can be accepted, or all of
 // space where that is not sure.  Acceptance looks at the point's barycentrics
 // alone, so the box holds only for a plane normal that is the triangle's own
@@ -1042,20 +1029,6 @@ __global__ void scene_scale_kernel(const splat_ftri_t* __restrict__ ftri, int64_
     if ((threadIdx.x & 31) == 0) atomicMax(scale, m);
 }
 
-__device__ __forceinline__ void padded_box(const float* p, float pad_abs, float pad_rel, float lo[3], float hi[3]) {
-    float tl[3], th[3];
-    for (int a = 0; a < 3; ++a) {
-        tl[a] = fminf(fminf(p[a], p[3 + a]), p[6 + a]);
-        th[a] = fmaxf(fmaxf(p[a], p[3 + a]), p[6 + a]);
-    }
-    const float dx = th[0] - tl[0], dy = th[1] - tl[1], dz = th[2] - tl[2];
-    const float pad = pad_abs + pad_rel * sqrtf(dx * dx + dy * dy + dz * dz);
-    for (int a = 0; a < 3; ++a) {
-        lo[a] = tl[a] - pad;
-        hi[a] = th[a] + pad;
-    }
-}
-
 __global__ void pack_hits_kernel(const splat_ftri_t* __restrict__ ftri, int64_t n_tris, TriHit* recs, TriBox* boxes,
                                  const unsigned* __restrict__ scale, const int32_t* __restrict__ order,
                                  int32_t* bvh_pos) {
@@ -1075,16 +1048,7 @@ __global__ void pack_hits_kernel(const splat_ftri_t* __restrict__ ftri, int64_t 
             boxes[j] = TriBox{make_float4(lo[0], lo[1], lo[2], 0.0f), make_float4(hi[0], hi[1], hi[2], 0.0f)};
             if (bvh_pos) bvh_pos[idx] = (int32_t)j;
         }
-        // merged boxes of 8 and of 32 records (a NaN box, which no ray enters, drops out)
-        for (int o = 1; o < 32; o <<= 1) {
-            for (int a = 0; a < 3; ++a) {
-                lo[a] = fminf(lo[a], __shfl_xor_sync(0xffffffffu, lo[a], o));
-                hi[a] = fmaxf(hi[a], __shfl_xor_sync(0xffffffffu, hi[a], o));
-            }
-            const TriBox m{make_float4(lo[0], lo[1], lo[2], 0.0f), make_float4(hi[0], hi[1], hi[2], 0.0f)};
-            if (o == 4 && (lane & 7) == 0 && j + 1 < n_tris) const_cast<TriBox*>(bb.box8)[j / 8] = m;
-            if (o == 16 && lane == 0) const_cast<TriBox*>(bb.box32)[j / 32] = m;
-        }
+        merge_boxes(bb, j, j + 1 < n_tris, lo, hi);
     }
     if (bvh_pos && blockIdx.x == 0 && threadIdx.x == 0) {
         bvh_pos[0] = 0;

@@ -729,6 +729,52 @@ __device__ __forceinline__ bool enters(const float4& lo, const float4& hi, const
     return (tmin <= tmax) & (tmax >= 0.0f) & (tmin <= best);
 }
 
+// ---------------------------------------------------------------------------
+// records and their boxes
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ TriHit pack_one(int32_t idx, F3 n, F3 a, F3 b, F3 c) {
+    TriHit h;
+    F3 v0 = c - a, v1 = b - a;
+    float dot00 = dot(v0, v0), dot01 = dot(v0, v1), dot11 = dot(v1, v1);
+    float invDenom = 1.0f / (dot00 * dot11 - dot01 * dot01);
+    h.n_nv = make_float4(n.x, n.y, n.z, dot(n, a));
+    h.a_idx = make_float4(a.x, a.y, a.z, __int_as_float(idx));
+    h.e0 = make_float4(v0.x, v0.y, v0.z, dot00);
+    h.e1 = make_float4(v1.x, v1.y, v1.z, dot11);
+    h.inv = make_float4(dot01, invDenom, 0.f, 0.f);
+    return h;
+}
+
+__device__ __forceinline__ void padded_box(const float* p, float pad_abs, float pad_rel, float lo[3], float hi[3]) {
+    float tl[3], th[3];
+    for (int a = 0; a < 3; ++a) {
+        tl[a] = fminf(fminf(p[a], p[3 + a]), p[6 + a]);
+        th[a] = fmaxf(fmaxf(p[a], p[3 + a]), p[6 + a]);
+    }
+    const float dx = th[0] - tl[0], dy = th[1] - tl[1], dz = th[2] - tl[2];
+    const float pad = pad_abs + pad_rel * sqrtf(dx * dx + dy * dy + dz * dz);
+    for (int a = 0; a < 3; ++a) {
+        lo[a] = tl[a] - pad;
+        hi[a] = th[a] + pad;
+    }
+}
+
+// Merged boxes of 8 and of 32 consecutive records: lane l of the warp holds
+// record j = 32 b + l (a NaN box, which no ray enters, drops out; lanes past
+// the end pass empty boxes).
+__device__ __forceinline__ void merge_boxes(const BruteBoxes& bb, int64_t j, bool valid, float lo[3], float hi[3]) {
+    const int lane = threadIdx.x & 31;
+    for (int o = 1; o < 32; o <<= 1) {
+        for (int a = 0; a < 3; ++a) {
+            lo[a] = fminf(lo[a], __shfl_xor_sync(0xffffffffu, lo[a], o));
+            hi[a] = fmaxf(hi[a], __shfl_xor_sync(0xffffffffu, hi[a], o));
+        }
+        const TriBox m{make_float4(lo[0], lo[1], lo[2], 0.0f), make_float4(hi[0], hi[1], hi[2], 0.0f)};
+        if (o == 4 && (lane & 7) == 0 && valid) const_cast<TriBox*>(bb.box8)[j / 8] = m;
+        if (o == 16 && lane == 0) const_cast<TriBox*>(bb.box32)[j / 32] = m;
+    }
+}
+
 // Closest hit of one ray over hit records in any order (the per-ray form of
 // the brute-force hitter; ties take the smaller index), each record behind
 // its padded box as in the tiled kernel.

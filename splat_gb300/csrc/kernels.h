@@ -193,8 +193,19 @@ cudaError_t launch_refit_trees(const RefitTrees& t, const TriHit* recs, const sp
 // as two-child and four-wide nodes with leaves of at most leaf_max triangles
 constexpr int kLbvhLeaf = 4;
 size_t lbvh_scratch_bytes(int64_t n_prims);
+// (each in an array of at least n_tris - 2 nodes, at its radix-tree index),
+// with the records, boxes, order and scale launch_pack_hits would write.
+struct LbvhOut {
+    BvhNode* nodes2;
+    Bvh4Node* nodes4;
+    int32_t* order;
+    TriHit* recs;
+    TriBox* boxes;
+    int32_t* bvh_pos;
+    unsigned* scale;
+};
 cudaError_t launch_lbvh_build(const splat_ftri_t* ftri, int64_t n_tris, int leaf_max, void* scratch,
-                              BvhNode* nodes2, Bvh4Node* nodes4, int32_t* order, int sm_count, cudaStream_t s);
+                              const LbvhOut& out, int sm_count, cudaStream_t s);
 
 // Coherent ray order (lbvh.cu): a permutation of the d_count active rays of
 // a SoA bounce buffer, grouped by (direction octant, BVH-order position of
