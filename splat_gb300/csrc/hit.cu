@@ -75,7 +75,7 @@ constexpr uint32_t kStallPolls = 64;
 // ---------------------------------------------------------------------------
 constexpr int kBruteThreads = 256;  // the n_tris drop-in kernel
 constexpr int kRPT = 2;
-constexpr int kTile = 64;  // records per tile of the n_tris drop-in kernel
+constexpr int kTile = 256;  // records per tile of the n_tris drop-in kernel
 constexpr int kStages = 4;
 
 // Every pair of a ray and a triangle is decided, but not one at a time: the
@@ -455,18 +455,55 @@ __device__ __forceinline__ TriBox ntris_box(const TriHit& h, F3 a, F3 b, F3 c, f
     return TriBox{make_float4(lx - pad, ly - pad, lz - pad, 0.f), make_float4(hx + pad, hy + pad, hz + pad, 0.f)};
 }
 
-// The tile's records get boxes as they are packed, merged over 8 and over the
-// 64 of a tile (ntris_box; a warp with a ray too far out for the boxes tests
-// every triangle).  40,000 rays, 5,123 triangles in an order without
-// locality: 583 -> 268 us (ncu, one GB300; before, a division and the full
-// test for every pair).
+// Ascending order of the block's 256 keys, one a thread (bitonic; strides
+// below a warp by shuffle, the others through shared memory).
+__device__ __forceinline__ uint32_t block_sort256(uint32_t key, uint32_t* s_key) {
+    const int i = threadIdx.x;
+#pragma unroll
+    for (int k = 2; k <= 256; k <<= 1) {
+#pragma unroll
+        for (int j = k >> 1; j; j >>= 1) {
+            uint32_t other;
+            if (j >= 32) {
+                __syncthreads();
+                s_key[i] = key;
+                __syncthreads();
+                other = s_key[i ^ j];
+            } else {
+                other = __shfl_xor_sync(0xffffffffu, key, j);
+            }
+            const bool up = (i & k) == 0, low = (i & j) == 0;
+            key = (low == up) ? min(key, other) : max(key, other);
+        }
+    }
+    return key;
+}
+
+__device__ __forceinline__ uint32_t spread8(uint32_t x) {  // 8 bits, two zeros between
+    x = (x | (x << 8)) & 0x0000f00fu;
+    x = (x | (x << 4)) & 0x000c30c3u;
+    return (x | (x << 2)) & 0x00249249u;
+}
+
+// A tile of 256 of the caller's records is packed, given boxes (ntris_box) and
+// put along a Morton curve of its own box, so that boxes merged over 8 and 32
+// of them are small whatever order the array has; a warp passes by those none
+// of its rays enters (a warp with a ray too far out for the boxes tests every
+// triangle).  Equal distances take the earlier record, as over the array's
+// order: pos is the record's place in its tile.  40,000 rays, 5,123
+// triangles: 583 -> 127 us (ncu, one GB300; a division and the full test for
+// every pair before; boxes in the array's order 268).
 __global__ void __launch_bounds__(kBruteThreads) hit_ntris_kernel(const splat_adray_t* __restrict__ rays,
                                                                    int64_t n_rays, const splat_ntri_t* __restrict__ nt,
                                                                    int64_t n_tris, int64_t per_split,
                                                                    unsigned long long* __restrict__ tmp) {
-    __shared__ TriHit tile[kTile];
+    static_assert(kTile == kBruteThreads && kTile == 256, "a record a thread");
+    constexpr int kWarps = kBruteThreads / 32;
+    __shared__ TriHit tile[kTile];  // inv.z: pos
     __shared__ TriBox box[kTile], box8[kTile / 8], box32[kTile / 32];
-    __shared__ float s_scale[kTile / 32];
+    __shared__ float s_ext[kWarps][7];
+    __shared__ uint32_t s_key[kTile];
+    __shared__ float s_scale;
     const float inf = __int_as_float(0x7f800000);
     RaySrc src{};
     src.aos = rays;
@@ -475,13 +512,14 @@ __global__ void __launch_bounds__(kBruteThreads) hit_ntris_kernel(const splat_ad
     const int64_t tb = (int64_t)blockIdx.y * per_split;
     const int64_t te = min(n_tris, tb + per_split);
     if (tb >= te) return;
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     HitRay ray[kRPT];
     float best[kRPT], inv[kRPT][3], oinv[kRPT][3];
-    int32_t bi[kRPT];
+    int32_t bi[kRPT], bpos[kRPT];
     float reach = 0.0f;  // largest |origin coordinate| over the warp
 #pragma unroll
     for (int r = 0; r < kRPT; ++r) {
-        const int64_t k = ray0 + threadIdx.x + (int64_t)r * kBruteThreads;
+        const int64_t k = ray0 + (wid * kRPT + r) * 32 + lane;
         ray[r] = k < n_rays ? load_hit_ray<true>(src, k) : HitRay{0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0};
         best[r] = k < n_rays ? inf : -inf;  // an idle lane's ray enters no box
         bi[r] = 1;
@@ -496,43 +534,90 @@ __global__ void __launch_bounds__(kBruteThreads) hit_ntris_kernel(const splat_ad
     reach = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(reach)));
     for (int64_t base = tb; base < te; base += kTile) {
         const int cnt = (int)min((int64_t)kTile, te - base);
-        if (threadIdx.x < kTile) {
-            const int j = threadIdx.x, lane = j & 31;
-            TriBox m{make_float4(inf, inf, inf, 0.f), make_float4(-inf, -inf, -inf, 0.f)};
-            float scale = inf;
-            if (j < cnt) {
-                const splat_ntri_t& q = nt[base + j];
-                const F3 a = f3(q.v[1]), b = f3(q.v[2]), c = f3(q.v[3]);
-                const TriHit h = pack_one(q.idx, f3(q.v[0]), a, b, c);
-                tile[j] = h;
-                m = ntris_box(h, a, b, c, scale);
-                box[j] = m;
-            }
-            for (int o = 1; o < 32; o <<= 1) {
-                m.lo.x = fminf(m.lo.x, __shfl_xor_sync(0xffffffffu, m.lo.x, o));
-                m.lo.y = fminf(m.lo.y, __shfl_xor_sync(0xffffffffu, m.lo.y, o));
-                m.lo.z = fminf(m.lo.z, __shfl_xor_sync(0xffffffffu, m.lo.z, o));
-                m.hi.x = fmaxf(m.hi.x, __shfl_xor_sync(0xffffffffu, m.hi.x, o));
-                m.hi.y = fmaxf(m.hi.y, __shfl_xor_sync(0xffffffffu, m.hi.y, o));
-                m.hi.z = fmaxf(m.hi.z, __shfl_xor_sync(0xffffffffu, m.hi.z, o));
-                scale = fminf(scale, __shfl_xor_sync(0xffffffffu, scale, o));
-                if (o == 4 && (lane & 7) == 0) box8[j / 8] = m;
-            }
-            if (lane == 0) {
-                box32[j / 32] = m;
-                s_scale[j / 32] = scale;
+        TriHit h;
+        TriBox m{make_float4(inf, inf, inf, 0.f), make_float4(-inf, -inf, -inf, 0.f)};
+        float scale = inf, c[3] = {0.f, 0.f, 0.f}, lo[3] = {inf, inf, inf}, hi[3] = {-inf, -inf, -inf};
+        if (tid < cnt) {
+            const splat_ntri_t& q = nt[base + tid];
+            const F3 v0 = f3(q.v[1]), v1 = f3(q.v[2]), v2 = f3(q.v[3]);
+            h = pack_one(q.idx, f3(q.v[0]), v0, v1, v2);
+            h.inv.z = __int_as_float(tid);
+            m = ntris_box(h, v0, v1, v2, scale);
+            c[0] = v0.x;
+            c[1] = v0.y;
+            c[2] = v0.z;
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                if (!(fabsf(c[a]) < inf)) c[a] = 0.0f;
+                lo[a] = hi[a] = c[a];
             }
         }
+        // the tile's extent and smallest scale
+        for (int o = 16; o; o >>= 1) {
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                lo[a] = fminf(lo[a], __shfl_xor_sync(0xffffffffu, lo[a], o));
+                hi[a] = fmaxf(hi[a], __shfl_xor_sync(0xffffffffu, hi[a], o));
+            }
+            scale = fminf(scale, __shfl_xor_sync(0xffffffffu, scale, o));
+        }
+        if (lane == 0) {
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                s_ext[wid][a] = lo[a];
+                s_ext[wid][3 + a] = hi[a];
+            }
+            s_ext[wid][6] = scale;
+        }
         __syncthreads();
+        uint32_t code = 0;
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            float l = inf, u = -inf;
+            for (int w = 0; w < kWarps; ++w) {
+                l = fminf(l, s_ext[w][a]);
+                u = fmaxf(u, s_ext[w][3 + a]);
+            }
+            const float f = u > l ? (c[a] - l) * (256.0f / (u - l)) : 0.0f;
+            code |= spread8((uint32_t)fminf(fmaxf(f, 0.0f), 255.0f)) << a;
+        }
+        if (tid == 0) {
+            float w = inf;
+            for (int i = 0; i < kWarps; ++i) w = fminf(w, s_ext[i][6]);
+            s_scale = w;
+        }
+        // sorted: the record that goes to slot tid; its owner learns the slot
+        const uint32_t key = block_sort256(tid < cnt ? (code << 8) | (uint32_t)tid : 0xffffff00u | (uint32_t)tid, s_key);
+        __syncthreads();
+        s_key[key & 255u] = (uint32_t)tid;
+        __syncthreads();
+        const int slot = (int)s_key[tid];
+        if (tid < cnt) tile[slot] = h;
+        box[slot] = m;
+        __syncthreads();
+        m = box[tid];
+        for (int o = 1; o < 32; o <<= 1) {
+            m.lo.x = fminf(m.lo.x, __shfl_xor_sync(0xffffffffu, m.lo.x, o));
+            m.lo.y = fminf(m.lo.y, __shfl_xor_sync(0xffffffffu, m.lo.y, o));
+            m.lo.z = fminf(m.lo.z, __shfl_xor_sync(0xffffffffu, m.lo.z, o));
+            m.hi.x = fmaxf(m.hi.x, __shfl_xor_sync(0xffffffffu, m.hi.x, o));
+            m.hi.y = fmaxf(m.hi.y, __shfl_xor_sync(0xffffffffu, m.hi.y, o));
+            m.hi.z = fmaxf(m.hi.z, __shfl_xor_sync(0xffffffffu, m.hi.z, o));
+            if (o == 4 && (lane & 7) == 0) box8[tid / 8] = m;
+        }
+        if (lane == 0) box32[wid] = m;
+        __syncthreads();
+        const bool all = !(reach <= kNtrisReach * s_scale);  // also a NaN reach
+#pragma unroll
+        for (int r = 0; r < kRPT; ++r) bpos[r] = -1;  // a best hit from an earlier tile wins ties
 #pragma unroll 1
-        for (int half = 0; half * 32 < cnt; ++half) {
-            const bool all = !(reach <= kNtrisReach * s_scale[half]);  // also a NaN reach
+        for (int part = 0; part * 32 < cnt; ++part) {
             bool some = all;
 #pragma unroll
-            for (int r = 0; r < kRPT; ++r) some |= enters(box32[half].lo, box32[half].hi, inv[r], oinv[r], best[r]);
+            for (int r = 0; r < kRPT; ++r) some |= enters(box32[part].lo, box32[part].hi, inv[r], oinv[r], best[r]);
             if (!__any_sync(0xffffffffu, some)) continue;
 #pragma unroll 1
-            for (int g = half * 4; g < half * 4 + 4 && g * 8 < cnt; ++g) {
+            for (int g = part * 4; g < part * 4 + 4 && g * 8 < cnt; ++g) {
                 bool in[kRPT];
                 some = false;
 #pragma unroll
@@ -549,15 +634,17 @@ __global__ void __launch_bounds__(kBruteThreads) hit_ntris_kernel(const splat_ad
                         if (!in[r] || !(all || enters(box[j].lo, box[j].hi, inv[r], oinv[r], best[r]))) continue;
                         float num, den;
                         if (!tri_candidate(q0, ray[r], best[r], num, den)) continue;
-                        const float4 q1 = tile[j].a_idx;
-                        const int32_t idx = __float_as_int(q1.w);
+                        const float4 q1 = tile[j].a_idx, q4 = tile[j].inv;
+                        const int32_t idx = __float_as_int(q1.w), pos = __float_as_int(q4.z);
                         bool inside;
-                        const float t = tri_t_from(num, den, q1, tile[j].e0, tile[j].e1, tile[j].inv, ray[r], inside);
+                        const float t = tri_t_from(num, den, q1, tile[j].e0, tile[j].e1, q4, ray[r], inside);
                         // next_hit_kernel6 (src/hitters.jl:183) has no i != 1 test: the
                         // sentinel's t is NaN and fails t > 0.
-                        if (inside & (t > 0.0f) & (idx != ray[r].ig) & (t < best[r])) {
+                        if (inside & (t > 0.0f) & (idx != ray[r].ig) &
+                            ((t < best[r]) | ((t == best[r]) & (pos < bpos[r])))) {
                             best[r] = t;
                             bi[r] = idx;
+                            bpos[r] = pos;
                         }
                     }
                 }
@@ -567,7 +654,7 @@ __global__ void __launch_bounds__(kBruteThreads) hit_ntris_kernel(const splat_ad
     }
 #pragma unroll
     for (int r = 0; r < kRPT; ++r) {
-        const int64_t k = ray0 + threadIdx.x + (int64_t)r * kBruteThreads;
+        const int64_t k = ray0 + (wid * kRPT + r) * 32 + lane;
         if (k < n_rays && bi[r] != 1) atomicMin(tmp + k, (unsigned long long)pack_argmin(best[r], (uint32_t)bi[r]));
     }
 }
@@ -581,7 +668,7 @@ cudaError_t launch_hit_brute_ntris(const splat_adray_t* rays, int64_t n_rays, co
     const int64_t rays_per_block = (int64_t)kBruteThreads * kRPT;
     const int64_t ray_blocks = (n_rays + rays_per_block - 1) / rays_per_block;
     int64_t splits = ((int64_t)sm_count * 4 + ray_blocks - 1) / ray_blocks;
-    const int64_t max_splits = (n_tris + 4 * kTile - 1) / (4 * kTile);
+    const int64_t max_splits = (n_tris + kTile - 1) / kTile;
     if (splits > max_splits) splits = max_splits;
     if (splits < 1) splits = 1;
     if (splits > 65535) splits = 65535;
