@@ -40,7 +40,9 @@ __device__ __forceinline__ void add_stats(splat_trace_stats_t* st, int diffuse, 
 // dropped); 2: camera (as trace, escaped rays queued unchanged for the sky).
 // MK >= 0: the material kind, fixed at compile time so that only that
 // material's optics is inlined (smaller code, no per-evaluation switch).
-template <int MODE, int MK>
+// PACKED: hits come as packed (t, index) words, and the survivors' words are
+// reset for the next bounce.
+template <int MODE, int MK, bool PACKED = false>
 __global__ void __launch_bounds__(kEvolveThreads) evolve_kernel(EvolveArgs A) {
     constexpr bool TRACE = MODE != 0;
     constexpr bool SKY = MODE == 2;
@@ -77,7 +79,8 @@ __global__ void __launch_bounds__(kEvolveThreads) evolve_kernel(EvolveArgs A) {
             EvolveView v{A.tris, A.n_tris, A.err, A.first_diffuse, A.material, A.seed, A.bounce,
                          A.force_rand, quirks, A.last != 0};
             if (MK >= 0) v.material.kind = MK;
-            const int fate = evolve_one<TRACE>(r, A.hit_idx[k], id, v, o, ih);
+            const int32_t hit = PACKED ? (int32_t)(uint32_t)A.hit_packed[k] : A.hit_idx[k];
+            const int fate = evolve_one<TRACE>(r, hit, id, v, o, ih);
             keep = fate == kFateKeep;
             dif = fate == kFateDiffuse;
             sky = SKY && fate == kFateInfinity;
@@ -120,7 +123,9 @@ __global__ void __launch_bounds__(kEvolveThreads) evolve_kernel(EvolveArgs A) {
         __syncthreads();
         const unsigned below = (1u << lane) - 1u;
         if (keep) {
-            store_ray(A.out, (int64_t)s_base + s_warp[wid] + __popc(kb & below), o, id);
+            const int64_t p = (int64_t)s_base + s_warp[wid] + __popc(kb & below);
+            store_ray(A.out, p, o, id);
+            if (PACKED) A.next_packed[p] = kNoHit;
         } else if (TRACE && dif) {
             store_ray(A.splat_q, (int64_t)s_dbase + s_wdif[wid] + __popc(db & below), o, id);
         } else if (SKY && sky) {
@@ -136,22 +141,22 @@ static int evolve_grid(int64_t cap, int sm_count) {
     return (int)(b < 1 ? 1 : b);
 }
 
-template <int MODE>
+template <int MODE, bool PACKED = false>
 static cudaError_t launch_evolve_mode(const EvolveArgs& a, int64_t cap, int sm_count, cudaStream_t s) {
     if (cap <= 0) return cudaSuccess;
     const int grid = evolve_grid(cap, sm_count);
     switch (a.material.kind) {
-        case SPLAT_MATERIAL_LINEAR_REF: evolve_kernel<MODE, SPLAT_MATERIAL_LINEAR_REF><<<grid, kEvolveThreads, 0, s>>>(a); break;
-        case SPLAT_MATERIAL_CAUCHY: evolve_kernel<MODE, SPLAT_MATERIAL_CAUCHY><<<grid, kEvolveThreads, 0, s>>>(a); break;
-        case SPLAT_MATERIAL_SELLMEIER: evolve_kernel<MODE, SPLAT_MATERIAL_SELLMEIER><<<grid, kEvolveThreads, 0, s>>>(a); break;
-        default: evolve_kernel<MODE, -1><<<grid, kEvolveThreads, 0, s>>>(a); break;
+        case SPLAT_MATERIAL_LINEAR_REF: evolve_kernel<MODE, SPLAT_MATERIAL_LINEAR_REF, PACKED><<<grid, kEvolveThreads, 0, s>>>(a); break;
+        case SPLAT_MATERIAL_CAUCHY: evolve_kernel<MODE, SPLAT_MATERIAL_CAUCHY, PACKED><<<grid, kEvolveThreads, 0, s>>>(a); break;
+        case SPLAT_MATERIAL_SELLMEIER: evolve_kernel<MODE, SPLAT_MATERIAL_SELLMEIER, PACKED><<<grid, kEvolveThreads, 0, s>>>(a); break;
+        default: evolve_kernel<MODE, -1, PACKED><<<grid, kEvolveThreads, 0, s>>>(a); break;
     }
     ++g_launches;
     return cudaGetLastError();
 }
 
 cudaError_t launch_evolve_trace(const EvolveArgs& a, int64_t cap, int sm_count, cudaStream_t s) {
-    return launch_evolve_mode<1>(a, cap, sm_count, s);
+    return a.hit_packed ? launch_evolve_mode<1, true>(a, cap, sm_count, s) : launch_evolve_mode<1>(a, cap, sm_count, s);
 }
 
 cudaError_t launch_evolve_camera(const EvolveArgs& a, int64_t cap, int sm_count, cudaStream_t s) {
@@ -387,17 +392,31 @@ cudaError_t launch_light_map(splat_adray_t* rays, int64_t n, const int32_t* hit_
     return cudaGetLastError();
 }
 
+// The step's counters into its statistics, by the last splat (rg.rays set):
+// every bounce is done by then.  They accumulate: a step run as several ray
+// ranges adds each range's counts into statistics cleared once.
+__device__ __forceinline__ void splat_stats(const SplatRange& rg, splat_trace_stats_t* st) {
+    if (!rg.rays || !st || blockIdx.x != 0) return;
+    const int i = threadIdx.x;
+    if (i < rg.depth)
+        atomicAdd(reinterpret_cast<unsigned long long*>(&st->rays_per_bounce[i]), (unsigned long long)rg.rays[i]);
+    else if (i == 8)
+        atomicAdd(reinterpret_cast<unsigned long long*>(&st->diffuse), (unsigned long long)*rg.end);
+    else if (i == 9 && *rg.err)
+        atomicOr(reinterpret_cast<unsigned long long*>(&st->error), (unsigned long long)(uint32_t)*rg.err);
+}
+
 // Queued diffuse rays -> light map, one lane per ray walking all its planes
 // (each plane's N x N sub-samples in the reference's order, x offset
 // fastest; runs of samples on the same texel add in a register before one
 // atomic).  Integer maps are bit-exact; float maps change only the order of
 // additions, which float atomics never fix anyway.
-__global__ void __launch_bounds__(256, 3) splat_kernel(RaySoA q, const int64_t* __restrict__ d_begin,
-                                                       const int64_t* __restrict__ d_count,
+__global__ void __launch_bounds__(256, 3) splat_kernel(RaySoA q, SplatRange rg,
                                                        const splat_ftri_t* __restrict__ tris, SplatParams sp,
                                                        splat_trace_stats_t* st) {
-    const int64_t k0 = d_begin ? *d_begin : 0;
-    const int64_t n = *d_count;
+    const int64_t k0 = rg.begin ? *rg.begin : 0;
+    const int64_t n = *rg.end;
+    splat_stats(rg, st);
     const int planes = sp.n_lambda > 0 ? sp.n_lambda : 1;
     int done = 0;
     for (int64_t k = k0 + blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < n;
@@ -413,13 +432,13 @@ __global__ void __launch_bounds__(256, 3) splat_kernel(RaySoA q, const int64_t* 
 // The same splat through the block's shared texel table: the block takes
 // 256 queued rays at a time and, plane by plane, sums their samples per
 // texel before one map atomic per distinct texel.
-__global__ void __launch_bounds__(256, 2) splat_agg_kernel(RaySoA q, const int64_t* __restrict__ d_begin,
-                                                           const int64_t* __restrict__ d_count,
+__global__ void __launch_bounds__(256, 2) splat_agg_kernel(RaySoA q, SplatRange rg,
                                                            const splat_ftri_t* __restrict__ tris, SplatParams sp,
                                                            splat_trace_stats_t* st) {
     __shared__ int32_t s_key[kAggSlots], s_val[kAggSlots];
-    const int64_t k0 = d_begin ? *d_begin : 0;
-    const int64_t n = *d_count;
+    const int64_t k0 = rg.begin ? *rg.begin : 0;
+    const int64_t n = *rg.end;
+    splat_stats(rg, st);
     const int planes = sp.n_lambda > 0 ? sp.n_lambda : 1;
     const TableSink sink{sp, s_key, s_val};
     table_clear(s_key, s_val);
@@ -446,16 +465,16 @@ __global__ void __launch_bounds__(256, 2) splat_agg_kernel(RaySoA q, const int64
     add_stats(st, 0, done);
 }
 
-cudaError_t launch_splat(const RaySoA& q, const int64_t* d_begin, const int64_t* d_count, const splat_ftri_t* tris,
-                         const SplatParams& sp, splat_trace_stats_t* stats, int sm_count, cudaStream_t s) {
+cudaError_t launch_splat(const RaySoA& q, const SplatRange& rg, const splat_ftri_t* tris, const SplatParams& sp,
+                         splat_trace_stats_t* stats, int sm_count, cudaStream_t s) {
     if (q.cap <= 0) return cudaSuccess;
     int64_t b = (q.cap + 255) / 256;
     const int64_t lim = (int64_t)sm_count * g_tune[SPLAT_TUNE_SPLAT_BLOCKS_PER_SM];
     if (b > lim) b = lim;
     if (g_tune[SPLAT_TUNE_SPLAT_AGGREGATE])
-        splat_agg_kernel<<<(int)(b < 1 ? 1 : b), 256, 0, s>>>(q, d_begin, d_count, tris, sp, stats);
+        splat_agg_kernel<<<(int)(b < 1 ? 1 : b), 256, 0, s>>>(q, rg, tris, sp, stats);
     else
-        splat_kernel<<<(int)(b < 1 ? 1 : b), 256, 0, s>>>(q, d_begin, d_count, tris, sp, stats);
+        splat_kernel<<<(int)(b < 1 ? 1 : b), 256, 0, s>>>(q, rg, tris, sp, stats);
     ++g_launches;
     return cudaGetLastError();
 }
@@ -468,30 +487,16 @@ cudaError_t launch_copy_count(const int64_t* src, int64_t* dst, cudaStream_t s) 
     return cudaGetLastError();
 }
 
-__global__ void stats_finish_kernel(const int64_t* counts, int depth, const int64_t* splat_count,
-                                    splat_trace_stats_t* st, const int32_t* err) {
-    // accumulates: a step run as several ray ranges adds each range's counts
-    // into statistics cleared once
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        for (int b = 0; b < depth && b < 8; ++b)
-            atomicAdd(reinterpret_cast<unsigned long long*>(&st->rays_per_bounce[b]), (unsigned long long)counts[b]);
-        if (splat_count) atomicAdd(reinterpret_cast<unsigned long long*>(&st->diffuse), (unsigned long long)*splat_count);
-        if (err) atomicOr(reinterpret_cast<unsigned long long*>(&st->error), (unsigned long long)(uint32_t)*err);
-    }
-}
-
-cudaError_t launch_stats_finish(const int64_t* counts, int depth, const int64_t* splat_count,
-                                splat_trace_stats_t* stats, const int32_t* err, cudaStream_t s) {
-    stats_finish_kernel<<<1, 32, 0, s>>>(counts, depth, splat_count, stats, err);
-    ++g_launches;
-    return cudaGetLastError();
-}
-
-__global__ void generate_soa_kernel(GenParams g, int64_t n, RaySoA out, int64_t* d_count) {
-    if (blockIdx.x == 0 && threadIdx.x == 0 && d_count) *d_count = n;
+// Also clears the step's n_counts counters, counts[0] the rays, and the packed
+// hits of the first bounce (packed, optional).
+__global__ void generate_soa_kernel(GenParams g, int64_t n, RaySoA out, int64_t* counts, int n_counts,
+                                    unsigned long long* packed) {
+    if (blockIdx.x == 0)
+        for (int i = threadIdx.x; i < n_counts; i += blockDim.x) counts[i] = i == 0 ? n : 0;
     for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < n; k += (int64_t)gridDim.x * blockDim.x) {
         const int64_t kid = g.ray_begin + k;
         store_ray(out, k, gen_ray(g, kid), (uint32_t)kid);
+        if (packed) packed[k] = kNoHit;
     }
 }
 
@@ -515,9 +520,11 @@ __global__ void __launch_bounds__(256) generate_aos_kernel(GenParams g, int64_t 
     }
 }
 
-cudaError_t launch_generate_soa(const GenParams& g, int64_t n, RaySoA out, int64_t* d_count, cudaStream_t s) {
+cudaError_t launch_generate_soa(const GenParams& g, int64_t n, RaySoA out, int64_t* counts, int n_counts,
+                                uint64_t* packed, cudaStream_t s) {
     if (n <= 0) return cudaSuccess;
-    generate_soa_kernel<<<evolve_grid(n, 152), 256, 0, s>>>(g, n, out, d_count);
+    generate_soa_kernel<<<evolve_grid(n, 152), 256, 0, s>>>(g, n, out, counts, n_counts,
+                                                            reinterpret_cast<unsigned long long*>(packed));
     ++g_launches;
     return cudaGetLastError();
 }

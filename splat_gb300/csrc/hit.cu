@@ -368,9 +368,10 @@ static void launch_brute_tiles(dim3 grid, cudaStream_t s, const RaySrc& rays, co
                                                                               hit_idx, hit_t, tmp, err, stall_tile);
 }
 
-cudaError_t launch_hit_brute(const RaySrc& rays, int64_t cap, const TriHit* recs, const TriBox* all_boxes,
-                             int64_t n_recs, int32_t* hit_idx, float* hit_t, uint64_t* tmp, int32_t* err, int sm_count,
-                             cudaStream_t s) {
+// packed: tmp holds kNoHit already and keeps the results.
+static cudaError_t brute_launch(const RaySrc& rays, int64_t cap, const TriHit* recs, const TriBox* all_boxes,
+                                int64_t n_recs, int32_t* hit_idx, float* hit_t, uint64_t* tmp, bool packed,
+                                int32_t* err, int sm_count, cudaStream_t s) {
     if (cap <= 0) return cudaSuccess;
     const BruteBoxes boxes = brute_boxes_of(all_boxes, n_recs);
     const int tile = g_tune[SPLAT_TUNE_BRUTE_TILE].load();
@@ -394,8 +395,8 @@ cudaError_t launch_hit_brute(const RaySrc& rays, int64_t cap, const TriHit* recs
     per_split = ((per_split + tile - 1) / tile) * tile;
     splits = (n_recs + per_split - 1) / per_split;
     if (splits < 1) splits = 1;
-    const bool use_tmp = splits > 1;
-    if (use_tmp) {
+    const bool use_tmp = packed || splits > 1;
+    if (use_tmp && !packed) {
         fill_u64_kernel<<<grid_for(cap, 256, sm_count, 8), 256, 0, s>>>((unsigned long long*)tmp, cap, rays.d_count,
                                                                         (unsigned long long)kNoHit);
         ++g_launches;
@@ -410,7 +411,7 @@ cudaError_t launch_hit_brute(const RaySrc& rays, int64_t cap, const TriHit* recs
         else
             launch_brute_tiles<64>(grid, s, rays, recs, boxes, n_recs, per_split, hit_idx, hit_t, t, err, stall_tile);
         ++g_launches;
-    } else {
+    } else if (!packed) {
         // no triangles: every ray misses
         miss_kernel<<<grid_for(cap, 256, sm_count, 8), 256, 0, s>>>(cap, rays.d_count, hit_idx, hit_t);
         ++g_launches;
@@ -418,8 +419,19 @@ cudaError_t launch_hit_brute(const RaySrc& rays, int64_t cap, const TriHit* recs
     }
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    if (use_tmp) return launch_unpack_hits(tmp, cap, rays.d_count, hit_idx, hit_t, s);
+    if (use_tmp && !packed) return launch_unpack_hits(tmp, cap, rays.d_count, hit_idx, hit_t, s);
     return cudaSuccess;
+}
+
+cudaError_t launch_hit_brute(const RaySrc& rays, int64_t cap, const TriHit* recs, const TriBox* boxes, int64_t n_recs,
+                             int32_t* hit_idx, float* hit_t, uint64_t* tmp, int32_t* err, int sm_count,
+                             cudaStream_t s) {
+    return brute_launch(rays, cap, recs, boxes, n_recs, hit_idx, hit_t, tmp, false, err, sm_count, s);
+}
+
+cudaError_t launch_hit_brute_packed(const RaySrc& rays, int64_t cap, const TriHit* recs, const TriBox* boxes,
+                                    int64_t n_recs, uint64_t* packed, int32_t* err, int sm_count, cudaStream_t s) {
+    return brute_launch(rays, cap, recs, boxes, n_recs, nullptr, nullptr, packed, true, err, sm_count, s);
 }
 
 // ---------------------------------------------------------------------------

@@ -159,6 +159,10 @@ __host__ __device__ inline BruteBoxes brute_boxes_of(const TriBox* all, int64_t 
 cudaError_t launch_hit_brute(const RaySrc& rays, int64_t cap, const TriHit* recs, const TriBox* boxes, int64_t n_recs,
                              int32_t* hit_idx, float* hit_t, uint64_t* tmp, int32_t* err, int sm_count,
                              cudaStream_t s);
+// the same with the results left as packed (t, index) words, which the caller
+// has reset to kNoHit
+cudaError_t launch_hit_brute_packed(const RaySrc& rays, int64_t cap, const TriHit* recs, const TriBox* boxes,
+                                    int64_t n_recs, uint64_t* packed, int32_t* err, int sm_count, cudaStream_t s);
 // brute force over the reference's n_tris array (Tuple{Int32,Tri})
 cudaError_t launch_hit_brute_ntris(const splat_adray_t* rays, int64_t n_rays, const splat_ntri_t* ntris,
                                    int64_t n_tris, uint64_t* tmp, int32_t* hit_idx, int sm_count, cudaStream_t s);
@@ -243,7 +247,10 @@ struct GenParams {
     uint32_t light_index;
     int64_t ray_begin;
 };
-cudaError_t launch_generate_soa(const GenParams& g, int64_t n, RaySoA out, int64_t* d_count, cudaStream_t s);
+// clears the step's n_counts counters (counts[0] = n) and, when given, the
+// packed hits of the first bounce
+cudaError_t launch_generate_soa(const GenParams& g, int64_t n, RaySoA out, int64_t* counts, int n_counts,
+                                uint64_t* packed, cudaStream_t s);
 cudaError_t launch_generate_aos(const GenParams& g, int64_t n, splat_adray_t* out, cudaStream_t s);
 // active rays to out (their number added to d_count), the others to idle
 // (d_idle); ids are the rays' slots
@@ -293,6 +300,8 @@ struct EvolveArgs {
     int32_t* aos_hit;       // plugin mode: and the hit they retired with, by slot
     RaySoA splat_q;         // trace mode: final-evolved diffuse rays (ignore = hit triangle)
     int64_t* splat_count;
+    const uint64_t* hit_packed;  // trace mode: hits as packed (t, index) words instead of hit_idx
+    uint64_t* next_packed;       // trace mode: the survivors' words for the next bounce, reset here
     RaySoA sky_q;           // camera mode: rays that escaped, unchanged
     int64_t* sky_count;
     int32_t tile_h;         // > 0: the input is a light grid of tile_h rows in column order, taken in its
@@ -346,22 +355,27 @@ cudaError_t launch_map_to_array(const int32_t* map, int64_t w, int64_t h, int64_
 
 // A whole trace step of at most kSmallStepRays rays in one launch (step.cu):
 // nodes4 null is the brute-force hitter; ea gives scene, material and draws
-// (its queues are unused).  stats accumulate, as launch_stats_finish leaves
-// them.
+// (its queues are unused).  stats accumulate, as the last splat leaves them.
 constexpr int64_t kSmallStepRays = 12288;
 constexpr int64_t kSmallStepBruteRecs = 1024;
 cudaError_t launch_small_step(const GenParams& gen, int64_t n, const Bvh4Node* nodes4, const TriHit* recs,
                               const TriBox* boxes, int64_t n_recs, const EvolveArgs& ea, int32_t depth,
                               const SplatParams& sp, splat_trace_stats_t* stats, cudaStream_t s);
 
-// light-map splat of the queued diffuse rays [*d_begin, *d_count) (d_begin
-// null: from 0)
-cudaError_t launch_splat(const RaySoA& q, const int64_t* d_begin, const int64_t* d_count, const splat_ftri_t* tris,
-                         const SplatParams& sp, splat_trace_stats_t* stats, int sm_count, cudaStream_t s);
+// light-map splat of the queued diffuse rays [*begin, *end) (begin null: from
+// 0).  The step's last splat also adds up its statistics: rays[b], the rays
+// entering bounce b + 1, for depth bounces, *end the diffuse rays, and the
+// scene's error word.
+struct SplatRange {
+    const int64_t *begin, *end;
+    const int64_t* rays;  // null: not the last
+    int depth;
+    const int32_t* err;
+};
+cudaError_t launch_splat(const RaySoA& q, const SplatRange& rg, const splat_ftri_t* tris, const SplatParams& sp,
+                         splat_trace_stats_t* stats, int sm_count, cudaStream_t s);
 // *dst = *src in stream order (a queue-length snapshot)
 cudaError_t launch_copy_count(const int64_t* src, int64_t* dst, cudaStream_t s);
-cudaError_t launch_stats_finish(const int64_t* counts, int depth, const int64_t* splat_count,
-                                splat_trace_stats_t* stats, const int32_t* err, cudaStream_t s);
 cudaError_t launch_unpack_hits(const uint64_t* tmp, int64_t n, const int64_t* d_count, int32_t* hit_idx,
                                float* hit_t, cudaStream_t s);
 
