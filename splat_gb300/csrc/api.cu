@@ -1795,7 +1795,14 @@ CameraParams camera_params(const splat_camera_t* cam, int64_t h, int64_t w, floa
     c.w = w;
     c.seed = seed;
     c.lambda = lambda;
-    c.cos45 = 1.0 / std::sqrt(2.0);
+    const double cos45 = 1.0 / std::sqrt(2.0);  // the reference's _COS_45 (src/geo.jl:13)
+    c.scale = ((double)h * cos45) / (double)cam->fov_half_sin;
+    c.p = 1.0 / c.scale;
+    for (int i = 0; i < 3; ++i) {
+        c.pr[i] = c.p * (double)cam->right[i];
+        c.pu[i] = c.p * (double)cam->up[i];
+        c.d[i] = cam->dir[i];
+    }
     return c;
 }
 
@@ -1878,8 +1885,7 @@ splat_status_t splat_camera_rays(const splat_camera_t* camera, int64_t height, i
     if (!d_rays) return fail(SPLAT_ERR_INVALID, "camera_rays: null output");
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     ProfScope ps(SPLAT_KERNEL_SHADE, st);
-    SPLAT_CUDA(launch_camera_aos(camera_params(camera, height, width, lambda, seed), height * width, d_rays,
-                                 sm_count_current(), st),
+    SPLAT_CUDA(launch_camera_aos(camera_params(camera, height, width, lambda, seed), height * width, d_rays, st),
                "camera rays");
     return SPLAT_OK;
 }
@@ -1955,7 +1961,7 @@ splat_status_t splat_shader_set_light_map(splat_shader_t* sh, const void* d_map,
         SPLAT_CUDA(copy_to_array(d_map, sh->map_w, sh->map_h, sh->planes, sh->map_arr, st), "light map -> array");
     } else if (accum == SPLAT_ACCUM_I32) {
         SPLAT_CUDA(launch_map_to_array(reinterpret_cast<const int32_t*>(d_map), sh->map_w, sh->map_h, sh->planes,
-                                       std::ldexp(1.0f, -frac_bits), sh->map_surf, sm_count_current(), st),
+                                       std::ldexp(1.0f, -frac_bits), sh->map_surf, st),
                    "light map -> array");
     } else {
         return fail(SPLAT_ERR_INVALID, "shader_set_light_map: unknown accumulation");
@@ -2031,8 +2037,7 @@ splat_status_t splat_render_camera_after(const splat_scene_t* scene, const splat
     SPLAT_CUDA(cudaMemsetAsync(d_rgb, 0, (size_t)P->height * P->width * 3 * sizeof(float), st), "clear image");
     {
         ProfScope ps(SPLAT_KERNEL_SHADE, st);
-        SPLAT_CUDA(launch_camera_soa(camera_params(&P->camera, ch, cw, P->lambda, P->seed), cnt, w.a, &w.counts[0],
-                                     sm, st),
+        SPLAT_CUDA(launch_camera_soa(camera_params(&P->camera, ch, cw, P->lambda, P->seed), cnt, w.a, &w.counts[0], st),
                    "camera rays");
     }
     EvolveArgs ea;
@@ -2077,10 +2082,14 @@ splat_status_t splat_render_camera_after(const splat_scene_t* scene, const splat
     }
     const ShadeParams sp =
         shade_params(shader, P->spectrum, &P->retina[0][0], P->n_lambda, P->upscale, P->height, d_rgb, SPLAT_MAX_LAMBDA);
+    {
+        // the skydome does not wait for the map
+        ProfScope ps(SPLAT_KERNEL_SHADE, st);
+        SPLAT_CUDA(launch_shade_sky(sky, sky_count, sp, cnt, sm, st), "shade sky");
+    }
     if (map_ready) SPLAT_CUDA(cudaStreamWaitEvent(st, reinterpret_cast<cudaEvent_t>(map_ready), 0), "wait for the map");
     ProfScope ps(SPLAT_KERNEL_SHADE, st);
-    SPLAT_CUDA(launch_shade_queues(w.q, &w.counts[kSplatCount], sky, sky_count, scene->d_ftri, sp, cnt, sm, st),
-               "shade");
+    SPLAT_CUDA(launch_shade_diffuse(w.q, &w.counts[kSplatCount], scene->d_ftri, sp, cnt, sm, st), "shade");
     return SPLAT_OK;
 }
 

@@ -325,7 +325,9 @@ struct CameraParams {
     int64_t h, w;      // camera grid (image / upscale)
     uint64_t seed;
     float lambda;
-    double cos45;      // 1 / sqrt(2), the reference's _COS_45 (src/geo.jl:13)
+    // of the whole grid: scale = h cos45 / fov_half_sin, p = 1 / scale, and the
+    // products p right, p up and dir in double
+    double scale, p, pr[3], pu[3], d[3];
 };
 struct ShadeParams {
     cudaTextureObject_t map_tex, sky_tex;
@@ -340,18 +342,18 @@ struct ShadeParams {
     float spectrum[SPLAT_MAX_LAMBDA];
     float retina[3][SPLAT_MAX_LAMBDA];
 };
-cudaError_t launch_camera_soa(const CameraParams& c, int64_t n, RaySoA out, int64_t* count, int sm_count,
-                              cudaStream_t s);
-cudaError_t launch_camera_aos(const CameraParams& c, int64_t n, splat_adray_t* out, int sm_count, cudaStream_t s);
-cudaError_t launch_shade_queues(const RaySoA& dq, const int64_t* d_count, const RaySoA& sq, const int64_t* s_count,
-                                const splat_ftri_t* tris, const ShadeParams& p, int64_t cap, int sm_count,
-                                cudaStream_t s);
+cudaError_t launch_camera_soa(const CameraParams& c, int64_t n, RaySoA out, int64_t* count, cudaStream_t s);
+cudaError_t launch_camera_aos(const CameraParams& c, int64_t n, splat_adray_t* out, cudaStream_t s);
+cudaError_t launch_shade_diffuse(const RaySoA& q, const int64_t* count, const splat_ftri_t* tris,
+                                 const ShadeParams& p, int64_t cap, int sm_count, cudaStream_t s);
+cudaError_t launch_shade_sky(const RaySoA& q, const int64_t* count, const ShadeParams& p, int64_t cap, int sm_count,
+                             cudaStream_t s);
 cudaError_t launch_shade_aos(splat_adray_t* rays, int64_t n, const int32_t* hit_idx, const splat_ftri_t* tris,
                              int64_t n_tris, int32_t* err, const ShadeParams& p, int sm_count, cudaStream_t s);
 cudaError_t launch_image_accumulate(float* out, const float* rgb, int64_t n, int32_t k, int sm_count,
                                     cudaStream_t s);
 cudaError_t launch_map_to_array(const int32_t* map, int64_t w, int64_t h, int64_t planes, float inv_scale,
-                                cudaSurfaceObject_t surf, int sm_count, cudaStream_t s);
+                                cudaSurfaceObject_t surf, cudaStream_t s);
 
 // A whole trace step of at most kSmallStepRays rays in one launch (step.cu):
 // nodes4 null is the brute-force hitter; ea gives scene, material and draws
