@@ -261,6 +261,72 @@ __device__ __forceinline__ void ray_to_aos(splat_adray_t& a, const RayState& r, 
     a.status = (uint8_t)status;
 }
 
+// Pairs of binary32 operations in one instruction (sm_100 and later), each
+// half rounded as the single operation rounds it.  The assembler contracts a
+// paired multiplication and the addition that takes it, .rn or not, so a
+// product is a fused multiply-add to -0, which is the same number; the -0
+// comes from constant memory, for one that the assembler knows it folds.
+static __constant__ float2 kNegZero2 = {-0.0f, -0.0f};
+__device__ __forceinline__ float2 dup2(float a) { return make_float2(a, a); }
+#define SPLAT_PAIR_OP(name, op)                                              \
+    __device__ __forceinline__ float2 name(float2 a, float2 b) {             \
+        float2 d;                                                            \
+        asm("{\n\t.reg .b64 x, y, w;\n\t"                                   \
+            "mov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\t" op            \
+            " w, x, y;\n\tmov.b64 {%0, %1}, w;\n\t}"                         \
+            : "=f"(d.x), "=f"(d.y)                                           \
+            : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));                       \
+        return d;                                                            \
+    }
+SPLAT_PAIR_OP(add2, "add.rn.f32x2")
+SPLAT_PAIR_OP(sub2, "sub.rn.f32x2")
+#undef SPLAT_PAIR_OP
+// fused: each half rounded as fmaf rounds it
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+    float2 d;
+    asm("{\n\t.reg .b64 x, y, z, w;\n\t"
+        "mov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tmov.b64 z, {%6, %7};\n\t"
+        "fma.rn.f32x2 w, x, y, z;\n\tmov.b64 {%0, %1}, w;\n\t}"
+        : "=f"(d.x), "=f"(d.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+    return d;
+}
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) { return fma2(a, b, kNegZero2); }
+
+// Two three-vectors, component by component.
+struct V2 {
+    float2 x, y, z;
+};
+__device__ __forceinline__ V2 pair3(F3 a, F3 b) {
+    return {make_float2(a.x, b.x), make_float2(a.y, b.y), make_float2(a.z, b.z)};
+}
+__device__ __forceinline__ V2 add2(V2 a, V2 b) { return {add2(a.x, b.x), add2(a.y, b.y), add2(a.z, b.z)}; }
+__device__ __forceinline__ V2 scale2(V2 a, float2 s) { return {mul2(a.x, s), mul2(a.y, s), mul2(a.z, s)}; }
+
+// -1 / sqrt(x) of both halves, square root and reciprocal each rounded to
+// nearest as 1.0f / sqrtf(x) rounds them.  One approximate inverse square
+// root y serves both: the remainder x - g^2 of g = x y, times y / 2, rounds
+// g to s = sqrt(x) (P. W. Markstein, IBM J. Res. Dev. 34, 1990), and the
+// residual e = 1 - s y, to second order, rounds y to 1 / s.  2^-36 breaks the
+// tie of the one significand for which that method is known to fail, all
+// ones.  Signs are chosen so that nothing is negated on its own.  A test
+// compares it with the plain form for every significand and both parities of
+// the exponent; a factor of 4 in x scales every term exactly while x is
+// within 2^-100 .. 2^100, and everything else (zero, subnormal, infinite,
+// NaN) takes the plain form.
+__device__ __forceinline__ float2 neg_inv_sqrt2(float2 x) {
+    if (!(x.x >= 0x1p-100f && x.y >= 0x1p-100f && x.x <= 0x1p100f && x.y <= 0x1p100f))
+        return make_float2(-(1.0f / sqrtf(x.x)), -(1.0f / sqrtf(x.y)));
+    float2 y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y.x) : "f"(x.x));
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y.y) : "f"(x.y));
+    const float2 g = mul2(x, y), nh = mul2(y, dup2(-0.5f));
+    const float2 s = fma2(fma2(g, g, mul2(x, dup2(-1.0f))), nh, g);
+    const float2 ny = add2(nh, nh);
+    const float2 e = fma2(s, ny, dup2(1.0f));
+    return fma2(fma2(e, add2(e, dup2(0x1p-36f)), e), ny, ny);
+}
+
 // Ray records through shared memory.  A record is 136 bytes, so a warp whose
 // lanes each read or write their own record touches 32 cache lines per
 // field, 34 fields long.  The kernels that go over whole arrays of records

@@ -411,9 +411,13 @@ __device__ __forceinline__ void splat_stats(const SplatRange& rg, splat_trace_st
 // fastest; runs of samples on the same texel add in a register before one
 // atomic).  Integer maps are bit-exact; float maps change only the order of
 // additions, which float atomics never fix anyway.
-__global__ void __launch_bounds__(256, 3) splat_kernel(RaySoA q, SplatRange rg,
-                                                       const splat_ftri_t* __restrict__ tris, SplatParams sp,
-                                                       splat_trace_stats_t* st) {
+// Instruction issue bounds it (splat_ray_plane_n).  96 registers at 20 warps
+// per SM: 24 warps at 80 registers spill more, 16 at 128 hide less latency
+// and made the step of 2^20 rays, 2 x 2 samples and 16 planes 2 % longer.
+constexpr int kSplatThreads = 128;
+__global__ void __launch_bounds__(kSplatThreads, 5) splat_kernel(RaySoA q, SplatRange rg,
+                                                                 const splat_ftri_t* __restrict__ tris,
+                                                                 SplatParams sp, splat_trace_stats_t* st) {
     const int64_t k0 = rg.begin ? *rg.begin : 0;
     const int64_t n = *rg.end;
     splat_stats(rg, st);
@@ -468,13 +472,19 @@ __global__ void __launch_bounds__(256, 2) splat_agg_kernel(RaySoA q, SplatRange 
 cudaError_t launch_splat(const RaySoA& q, const SplatRange& rg, const splat_ftri_t* tris, const SplatParams& sp,
                          splat_trace_stats_t* stats, int sm_count, cudaStream_t s) {
     if (q.cap <= 0) return cudaSuccess;
-    int64_t b = (q.cap + 255) / 256;
-    const int64_t lim = (int64_t)sm_count * g_tune[SPLAT_TUNE_SPLAT_BLOCKS_PER_SM];
+    const bool agg = g_tune[SPLAT_TUNE_SPLAT_AGGREGATE] != 0;
+    const int threads = agg ? 256 : kSplatThreads;
+    int64_t b = (q.cap + threads - 1) / threads;
+    // the knob counts 160 threads a block for the one without a table: its
+    // default of 8 is two full waves of 10 blocks of 128 (1.287 ms; 8 blocks
+    // 1.299, 16 blocks 1.292, and 521, 521, 529 us for the water surface)
+    int64_t lim = (int64_t)sm_count * g_tune[SPLAT_TUNE_SPLAT_BLOCKS_PER_SM];
+    if (!agg) lim = lim * 160 / kSplatThreads;
     if (b > lim) b = lim;
-    if (g_tune[SPLAT_TUNE_SPLAT_AGGREGATE])
-        splat_agg_kernel<<<(int)(b < 1 ? 1 : b), 256, 0, s>>>(q, rg, tris, sp, stats);
+    if (agg)
+        splat_agg_kernel<<<(int)b, threads, 0, s>>>(q, rg, tris, sp, stats);
     else
-        splat_kernel<<<(int)(b < 1 ? 1 : b), 256, 0, s>>>(q, rg, tris, sp, stats);
+        splat_kernel<<<(int)b, threads, 0, s>>>(q, rg, tris, sp, stats);
     ++g_launches;
     return cudaGetLastError();
 }

@@ -120,18 +120,6 @@ __device__ __forceinline__ float min3f(float a, float b, float c) {
     return d;
 }
 
-// Two binary32 fused multiply-adds in one instruction (sm_100 and later),
-// each rounded as fmaf rounds it.
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
-    float2 d;
-    asm("{\n\t.reg .b64 x, y, z, w;\n\t"
-        "mov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tmov.b64 z, {%6, %7};\n\t"
-        "fma.rn.f32x2 w, x, y, z;\n\tmov.b64 {%0, %1}, w;\n\t}"
-        : "=f"(d.x), "=f"(d.y)
-        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
-    return d;
-}
-
 // Entry and exit distances of a ray through the four child boxes of a
 // node.  The slab planes are picked by the signs of the inverse direction
 // (ix < 0: the near x plane is hi, else lo), through the addresses of the
