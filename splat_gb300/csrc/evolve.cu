@@ -14,6 +14,8 @@
 // (runs of samples on one texel are summed in a register first), which makes
 // the map independent of ray order and bit-exact run to run.  Float maps use
 // plain float atomics, as the reference does.
+#include <algorithm>
+
 #include "kernels.h"
 #include "optics.cuh"
 
@@ -297,20 +299,25 @@ cudaError_t launch_partition(splat_adray_t* rays, int64_t n, int64_t* counts, in
 // and triangle index, 28 words of its 34), so warps splat with all lanes
 // busy.  What it was bound by before: one ray at a time per warp, its 27
 // values and triangle broadcast to the lanes that held its samples.  2^18
-// rays, 12 planes, 2 x 2 offsets: 311.7 -> 154.3 us (ncu, one GB300).
-__global__ void __launch_bounds__(kEvolveThreads, 2) light_map_kernel(splat_adray_t* rays, int64_t n,
-                                                                      const int32_t* __restrict__ hit_idx,
-                                                                      const splat_ftri_t* __restrict__ tris,
-                                                                      int64_t n_tris, int32_t* err, SplatParams sp) {
-    constexpr int kWarps = kEvolveThreads / 32;
+// rays, 12 planes, 2 x 2 offsets: 311.7 -> 137.6 us (ncu, one GB300).  A block
+// of 128 for every 128 records, four at a time per SM: the whole frame of
+// those rays takes 632 us with blocks of 256 that go over the records in two
+// or more turns, and 617 so.
+constexpr int kMapThreads = 128;
+
+__global__ void __launch_bounds__(kMapThreads, 4) light_map_kernel(splat_adray_t* rays, int64_t n,
+                                                                   const int32_t* __restrict__ hit_idx,
+                                                                   const splat_ftri_t* __restrict__ tris,
+                                                                   int64_t n_tris, int32_t* err, SplatParams sp) {
+    constexpr int kWarps = kMapThreads / 32;
     __shared__ AosTile s_tile[kWarps];
     __shared__ int s_cnt[kWarps];
-    float* pool = reinterpret_cast<float*>(s_tile);  // [plane][kEvolveThreads], kPlanes + 1 planes
-    static_assert(sizeof(s_tile) >= sizeof(float) * (kPlanes + 1) * kEvolveThreads, "pool fits the tiles");
+    float* pool = reinterpret_cast<float*>(s_tile);  // [plane][kMapThreads], kPlanes + 1 planes
+    static_assert(sizeof(s_tile) >= sizeof(float) * (kPlanes + 1) * kMapThreads, "pool fits the tiles");
     const int lane = lane_id(), wid = threadIdx.x >> 5;
     AosTile& tile = s_tile[wid];
     const int planes = sp.n_lambda > 0 ? sp.n_lambda : 1;
-    for (int64_t base = (int64_t)blockIdx.x * kEvolveThreads; base < n; base += (int64_t)gridDim.x * kEvolveThreads) {
+    for (int64_t base = (int64_t)blockIdx.x * kMapThreads; base < n; base += (int64_t)gridDim.x * kMapThreads) {
         const int64_t wbase = base + 32 * wid, k = wbase + lane;
         bool dif = false;
         RayState o;
@@ -345,7 +352,7 @@ __global__ void __launch_bounds__(kEvolveThreads, 2) light_map_kernel(splat_adra
             before += w < wid ? c : 0;
             total += c;
         }
-        const RaySoA q{pool, nullptr, nullptr, nullptr, kEvolveThreads};
+        const RaySoA q{pool, nullptr, nullptr, nullptr, kMapThreads};
         if (dif) {
             const int p = before + __popc(db & ((1u << lane) - 1u));
             st3(q.f, q.cap, 0, p, o.pos);
@@ -387,7 +394,8 @@ __global__ void __launch_bounds__(kEvolveThreads, 2) light_map_kernel(splat_adra
 cudaError_t launch_light_map(splat_adray_t* rays, int64_t n, const int32_t* hit_idx, const splat_ftri_t* tris,
                              int64_t n_tris, int32_t* err, const SplatParams& sp, int sm_count, cudaStream_t s) {
     if (n <= 0) return cudaSuccess;
-    light_map_kernel<<<evolve_grid(n, sm_count), kEvolveThreads, 0, s>>>(rays, n, hit_idx, tris, n_tris, err, sp);
+    const int64_t b = std::min<int64_t>((n + kMapThreads - 1) / kMapThreads, (int64_t)sm_count * 64);
+    light_map_kernel<<<(int)b, kMapThreads, 0, s>>>(rays, n, hit_idx, tris, n_tris, err, sp);
     ++g_launches;
     return cudaGetLastError();
 }
