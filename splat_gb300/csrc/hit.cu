@@ -1045,7 +1045,11 @@ static void launch_bvh4_form(const RaySrc& rays, int64_t cap, const Bvh4View& bv
             hit_bvh4_refill_kernel<false><<<grid, kBvhThreads, 0, s>>>(rays, bvh, hit_idx, hit_t, err, m);
         return;
     }
-    const int grid = grid_of(reinterpret_cast<const void*>(hit_bvh4_kernel<false, COUNT>));
+    // a caller's records have no order, and their long rays hold up the rest of
+    // a warp's turns: twice the blocks, so that more start on their own
+    // (350,000 records, four calls in a bounce loop of the caller: 660 -> 647 us)
+    const int grid = rays.aos && !rays.fetch ? grid_for(cap, kBvhThreads, sm_count, 2 * knob)
+                                             : grid_of(reinterpret_cast<const void*>(hit_bvh4_kernel<false, COUNT>));
     if (rays.aos)
         hit_bvh4_kernel<true, COUNT><<<grid, kBvhThreads, 0, s>>>(rays, bvh, hit_idx, hit_t, err);
     else
