@@ -859,12 +859,20 @@ __global__ void __launch_bounds__(kBvhThreads) hit_bvh_kernel(RaySrc src, BvhVie
     });
 }
 
+// A caller's records come without a work counter and in no order, and a long
+// ray holds up the rays that its warp takes after it: they get four times the
+// blocks of the knob, so that most warps take one turn.  982,000 scattered
+// rays on a sphere, two-wide tree: 351 -> 306 us; 350,000 records, four calls
+// of the caller's bounce loop, four-wide: 660 -> 647 us.
+constexpr int kAosGrid = 4;
+
 cudaError_t launch_hit_bvh(const RaySrc& rays, int64_t cap, const BvhView& bvh, int32_t* hit_idx, float* hit_t,
                            int32_t* err, int sm_count, cudaStream_t s) {
     if (cap <= 0) return cudaSuccess;
     const int grid = rays.fetch ? resident_grid(reinterpret_cast<const void*>(hit_bvh_kernel<false>), cap, sm_count,
                                                 kBvhThreads, g_tune[SPLAT_TUNE_BVH_BLOCKS_PER_SM])
-                                : grid_for(cap, kBvhThreads, sm_count, g_tune[SPLAT_TUNE_BVH_BLOCKS_PER_SM]);
+                                : grid_for(cap, kBvhThreads, sm_count,
+                                           (rays.aos ? kAosGrid : 1) * g_tune[SPLAT_TUNE_BVH_BLOCKS_PER_SM]);
     if (rays.aos)
         hit_bvh_kernel<true><<<grid, kBvhThreads, 0, s>>>(rays, bvh, hit_idx, hit_t, err);
     else
@@ -1045,10 +1053,7 @@ static void launch_bvh4_form(const RaySrc& rays, int64_t cap, const Bvh4View& bv
             hit_bvh4_refill_kernel<false><<<grid, kBvhThreads, 0, s>>>(rays, bvh, hit_idx, hit_t, err, m);
         return;
     }
-    // a caller's records have no order, and their long rays hold up the rest of
-    // a warp's turns: twice the blocks, so that more start on their own
-    // (350,000 records, four calls in a bounce loop of the caller: 660 -> 647 us)
-    const int grid = rays.aos && !rays.fetch ? grid_for(cap, kBvhThreads, sm_count, 2 * knob)
+    const int grid = rays.aos && !rays.fetch ? grid_for(cap, kBvhThreads, sm_count, kAosGrid * knob)
                                              : grid_of(reinterpret_cast<const void*>(hit_bvh4_kernel<false, COUNT>));
     if (rays.aos)
         hit_bvh4_kernel<true, COUNT><<<grid, kBvhThreads, 0, s>>>(rays, bvh, hit_idx, hit_t, err);
