@@ -49,9 +49,12 @@ __host__ __device__ __forceinline__ D operator/(float a, D b) {
     float q = a / b.v;
     return {q, -(q / b.v) * b.d};
 }
+// The reference's 1 / (2 s), as half of the 1 / s that normalize needs anyway:
+// a square root of binary32 is far from the ends of the range, so the factor
+// of two is exact on either side of the rounding.
 __host__ __device__ __forceinline__ D dsqrt(D a) {
     float s = sqrtf(a.v);
-    return {s, (1.0f / (2.0f * s)) * a.d};
+    return {s, (0.5f * (1.0f / s)) * a.d};
 }
 __host__ __device__ __forceinline__ float dsqrt(float a) { return sqrtf(a); }
 __host__ __device__ __forceinline__ float val(float a) { return a; }

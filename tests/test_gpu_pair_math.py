@@ -1,8 +1,9 @@
 """The splat's paired arithmetic rounds as the plain operations do: inverse
 square roots for every significand and both parities of the exponent, at
 scales over the whole range of binary32 and for zeros, subnormals, infinities
-and NaN; sums, differences and products of pairs over random bit patterns, products
-not contracted into the sums that take them."""
+and NaN, the partial of a square root likewise; sums, differences and products
+of pairs over random bit patterns, products not contracted into the sums that
+take them."""
 import subprocess
 
 import pytest
@@ -23,6 +24,8 @@ __device__ void check(float x, float y) {
     const float2 g = neg_inv_sqrt2(make_float2(x, y));
     if (!same(g.x, -(1.0f / sqrtf(x)))) atomicAdd(&bad[0], 1ull);
     if (!same(g.y, -(1.0f / sqrtf(y)))) atomicAdd(&bad[0], 1ull);
+    const float root = sqrtf(x);  // the reference's partial of a square root
+    if (!same(dsqrt(D{x, 1.0f}).d, 1.0f / (2.0f * root))) atomicAdd(&bad[0], 1ull);
 }
 // i: the significand and the exponent's lowest bit; e: the scale
 __global__ void inv_sqrt(int e) {
