@@ -432,8 +432,12 @@ __device__ __forceinline__ void splat_stats(const SplatRange& rg, splat_trace_st
 // additions, which float atomics never fix anyway.
 // Instruction issue bounds it (splat_ray_plane_n).  96 registers at 20 warps
 // per SM: 24 warps at 80 registers spill more, 16 at 128 hide less latency
-// and made the step of 2^20 rays, 2 x 2 samples and 16 planes 2 % longer.
+// and made the step of 2^20 rays, 2 x 2 samples and 16 planes 2 % longer.  One
+// kernel for each of 1 x 1, 2 x 2 and other samples and each map type leaves
+// more registers to the one that runs: that step 1.263 -> 1.258 ms, the water
+// surface 515 -> 511 us.
 constexpr int kSplatThreads = 128;
+template <int ND, int ACCUM>
 __global__ void __launch_bounds__(kSplatThreads, 5) splat_kernel(RaySoA q, SplatRange rg,
                                                                  const splat_ftri_t* __restrict__ tris,
                                                                  SplatParams sp, splat_trace_stats_t* st) {
@@ -441,15 +445,25 @@ __global__ void __launch_bounds__(kSplatThreads, 5) splat_kernel(RaySoA q, Splat
     const int64_t n = *rg.end;
     splat_stats(rg, st);
     const int planes = sp.n_lambda > 0 ? sp.n_lambda : 1;
+    const DirectSink<SplatParams, ACCUM> sink{sp};
     int done = 0;
     for (int64_t k = k0 + blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < n;
          k += (int64_t)gridDim.x * blockDim.x) {
         const RayState r = load_ray(q, k);
         const Tri T = load_tri(tris, r.ignore);
         const TriUV quv = tri_uv(T);
-        for (int il = 0; il < planes; ++il) done += splat_ray_plane(sp, r, T, quv, il);
+        for (int il = 0; il < planes; ++il) done += splat_ray_plane_n<ND>(sp, r, T, quv, il, sink);
     }
     add_stats(st, 0, done);
+}
+
+template <int ND>
+static void launch_splat_nd(int grid, const RaySoA& q, const SplatRange& rg, const splat_ftri_t* tris,
+                            const SplatParams& sp, splat_trace_stats_t* stats, cudaStream_t s) {
+    if (sp.accum == SPLAT_ACCUM_I32)
+        splat_kernel<ND, SPLAT_ACCUM_I32><<<grid, kSplatThreads, 0, s>>>(q, rg, tris, sp, stats);
+    else
+        splat_kernel<ND, SPLAT_ACCUM_F32><<<grid, kSplatThreads, 0, s>>>(q, rg, tris, sp, stats);
 }
 
 // The same splat through the block's shared texel table: the block takes
@@ -502,8 +516,12 @@ cudaError_t launch_splat(const RaySoA& q, const SplatRange& rg, const splat_ftri
     if (b > lim) b = lim;
     if (agg)
         splat_agg_kernel<<<(int)b, threads, 0, s>>>(q, rg, tris, sp, stats);
+    else if (sp.n_delta == 2)
+        launch_splat_nd<2>((int)b, q, rg, tris, sp, stats, s);
+    else if (sp.n_delta == 1)
+        launch_splat_nd<1>((int)b, q, rg, tris, sp, stats, s);
     else
-        splat_kernel<<<(int)b, threads, 0, s>>>(q, rg, tris, sp, stats);
+        launch_splat_nd<0>((int)b, q, rg, tris, sp, stats, s);
     ++g_launches;
     return cudaGetLastError();
 }

@@ -384,19 +384,24 @@ __device__ __forceinline__ SplatView splat_view(const SplatParams& sp) {
 }
 
 template <class P>
-__device__ __forceinline__ void flush_texel(const P& sp, int32_t off, int32_t vi, float vf) {
+__device__ __forceinline__ void flush_texel(const P& sp, int32_t accum, int32_t off, int32_t vi, float vf) {
     if (off < 0) return;
-    if (sp.accum == SPLAT_ACCUM_I32)
+    if (accum == SPLAT_ACCUM_I32)
         atomicAdd(reinterpret_cast<int*>(sp.map) + off, vi);
     else
         atomicAdd(reinterpret_cast<float*>(sp.map) + off, vf);
 }
 
-// Sends a texel's partial sum straight to the map.
-template <class P>
+// Sends a texel's partial sum straight to the map.  A sink's kAccum is the
+// map's type where it is known at compile time (the other type's sums are then
+// not kept), -1 where sp.accum says it.
+template <class P, int ACCUM = -1>
 struct DirectSink {
+    static constexpr int kAccum = ACCUM;
     const P& sp;
-    __device__ __forceinline__ void operator()(int32_t off, int32_t vi, float vf) const { flush_texel(sp, off, vi, vf); }
+    __device__ __forceinline__ void operator()(int32_t off, int32_t vi, float vf) const {
+        flush_texel(sp, ACCUM < 0 ? sp.accum : ACCUM, off, vi, vf);
+    }
 };
 
 // Block-level texel aggregation.  Samples of the rays a block holds are
@@ -413,6 +418,7 @@ constexpr int kAggSlots = 1 << kAggLog2;
 constexpr int kAggProbes = 16;
 
 struct TableSink {
+    static constexpr int kAccum = -1;
     const SplatParams& sp;
     int32_t* keys;  // shared, -1 = empty
     int32_t* vals;  // shared, int32 sum or float bits
@@ -428,13 +434,14 @@ struct TableSink {
             }
             h = (h + 1) & (kAggSlots - 1);
         }
-        flush_texel(sp, off, vi, vf);
+        flush_texel(sp, sp.accum, off, vi, vf);
     }
 };
 
 // The table of a block whose rays splat into different maps (the batch
 // engine): keyed by the texel's address, its low bit set for float maps.
 struct AddrTableSink {
+    static constexpr int kAccum = -1;
     const SplatParams& sp;
     unsigned long long* keys;  // shared, 0 = empty
     int32_t* vals;
@@ -453,7 +460,7 @@ struct AddrTableSink {
             }
             h = (h + 1) & (kAggSlots - 1);
         }
-        flush_texel(sp, off, vi, vf);
+        flush_texel(sp, sp.accum, off, vi, vf);
     }
 };
 
@@ -490,7 +497,7 @@ __device__ __forceinline__ void table_flush(const SplatParams& sp, int32_t* keys
         const int32_t k = keys[i];
         if (k >= 0) {
             const int32_t v = vals[i];
-            flush_texel(sp, k, v, __int_as_float(v));
+            flush_texel(sp, sp.accum, k, v, __int_as_float(v));
             keys[i] = -1;
             vals[i] = 0;
         }
@@ -555,15 +562,16 @@ __device__ __forceinline__ int splat_ray_plane_n(const P& sp, const RayState& r,
             const float2 inv = neg_inv_sqrt2(make_float2(dot(nn, nn), dot(dir, dir)));
             const float inten = fabsf(dot(nn * inv.x, dir * inv.y));
             ++done;
-            const int32_t vi = __float2int_rn(inten * sp.scale);
+            const int32_t vi = Sink::kAccum == SPLAT_ACCUM_F32 ? 0 : __float2int_rn(inten * sp.scale);
+            const float vf = Sink::kAccum == SPLAT_ACCUM_I32 ? 0.0f : inten;
             if (off == run_off) {
                 run_i += vi;
-                run_f += inten;
+                run_f += vf;
             } else {
                 sink(run_off, run_i, run_f);
                 run_off = off;
                 run_i = vi;
-                run_f = inten;
+                run_f = vf;
             }
         }
     }
