@@ -552,15 +552,6 @@ static SplatParams make_splat(const float* spectrum, int32_t n_lambda, int64_t u
     // upres(N), src/alg_types.jl:108
     for (int k = 1; k <= sp.n_delta; ++k)
         sp.deltas[k - 1] = ((float)k / (float)sp.n_delta - 0.5f) - (1.0f / (2.0f * (float)sp.n_delta));
-    sp.n_samples = (n_lambda > 0 ? n_lambda : 1) * sp.n_delta * sp.n_delta;
-    // splat kernel: one lane per (ray, plane)
-    const int planes = n_lambda > 0 ? n_lambda : 1;
-    int l2 = 0;
-    while ((1 << l2) < planes && l2 < 5) ++l2;
-    sp.lanes_log2 = l2;
-    sp.chunks = (planes + (1 << l2) - 1) >> l2;
-    sp.inv_nd = 1.0f / (float)sp.n_delta;
-    sp.inv_nd2 = 1.0f / (float)(sp.n_delta * sp.n_delta);
     return sp;
 }
 
