@@ -603,6 +603,9 @@ splat_status_t splat_run_evolution(const splat_scene_t* scene, int32_t hitter, s
         RaySrc src{cur.f, cur.ignore, cur.cap, nullptr, &w.counts[b - 1], 0,
                    reinterpret_cast<unsigned long long*>(&w.counts[kFetchBase + b]), packet_for(b)};
         src.few = b > 1 ? 1 : 0;
+        if (b == 1 && src.packet == 1 && g_tune[SPLAT_TUNE_BVH_PACKET] == 1 &&
+            !packet_density(n_rays, scene->n_recs, kStripRaysPerTri))
+            src.packet = 0;
         splat_status_t rc = hit_any(scene, hitter, src, n_rays, w.hit, nullptr, w.tmp, st);
         if (rc != SPLAT_OK) return rc;
         ea.in = cur;
@@ -2053,7 +2056,8 @@ splat_status_t splat_render_camera_after(const splat_scene_t* scene, const splat
         // camera rays are the sub-sample grid's columns in order: first-bounce
         // packets take 8 x 4 tiles of it
         if (b == 1 && ch <= (int64_t)kGridTileMaxRows) src.tile_h = (int32_t)ch;
-        if (b == 1 && src.packet == 1 && g_tune[SPLAT_TUNE_BVH_PACKET] == 1 && !packet_density(cnt, scene->n_recs))
+        if (b == 1 && src.packet == 1 && g_tune[SPLAT_TUNE_BVH_PACKET] == 1 &&
+            !packet_density(cnt, scene->n_recs, kCameraRaysPerTri))
             src.packet = 0;
         rc = hit_any(scene, P->hitter, src, cnt, w.hit, nullptr, w.tmp, st);
         if (rc != SPLAT_OK) return rc;

@@ -44,8 +44,24 @@ struct RaySrc {
 //   displaced sphere, 20,482   1.6 116/132   3.2 122/120   6.4 136/123   12.8 174/135
 //   sponge, 96,012             0.7  68/72    1.4  84/90    2.7 112/107   10.9 270/241
 constexpr float kPacketRaysPerTri = 2.5f;
-__host__ __device__ inline bool packet_density(int64_t grid_rays, int64_t n_recs) {
-    return (float)grid_rays >= kPacketRaysPerTri * (float)n_recs;
+// A caller's records come in their own order, at best columns of a grid: a
+// packet is a strip of 32 x 1.  Measured likewise, us a frame of two bounces
+// from a light, or a camera pass, lane / packets:
+//   light, sphere, 81,922    0.8 281/328   1.6 355/439   3.2 507/538   6.4 719/706   12.8 1172/1112
+//   light, displaced, 20,482 3.2 270/273   6.3 323/319   12.8 458/427
+//   light, sponge, 96,012    1.4 296/317   2.7 473/488   5.5 756/776   10.9 1306/1313  21.8 2376/2370
+//   camera, sphere, 81,922   0.7 308/430   1.8 469/602   3.3 578/656
+//   camera, displaced, 20,482  2.8 261/290   7.2 397/425   13 518/515
+constexpr float kStripRaysPerTri = 6.0f;
+// The fused camera pass's rays come in tiles again, but from one point towards
+// the whole view; a frame of two bounces, lane / packets:
+//   displaced, 81,922   2.8 363/396   3.6 412/404   6.3 458/462
+//   displaced, 20,482   2.8 180/186   4.3 223/219   11.2 266/260
+//   sphere, 20,482      4.3 218/207   8.8 240/230
+constexpr float kCameraRaysPerTri = 3.2f;
+__host__ __device__ inline bool packet_density(int64_t grid_rays, int64_t n_recs,
+                                               float per_tri = kPacketRaysPerTri) {
+    return (float)grid_rays >= per_tri * (float)n_recs;
 }
 
 // Which traversal a warp of four-wide BVH rays takes, from
