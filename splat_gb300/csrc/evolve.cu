@@ -15,6 +15,7 @@
 // the map independent of ray order and bit-exact run to run.  Float maps use
 // plain float atomics, as the reference does.
 #include <algorithm>
+#include <type_traits>
 
 #include "kernels.h"
 #include "optics.cuh"
@@ -303,6 +304,24 @@ cudaError_t launch_partition(splat_adray_t* rays, int64_t n, int64_t* counts, in
     return cudaGetLastError();
 }
 
+// go(N, ACCUM) with the splat's sample count, 1, 2 or 0 (any), and map type as
+// compile-time constants.
+template <class Go>
+static void by_form(const SplatParams& sp, const Go& go) {
+    auto typed = [&](auto nd) {
+        if (sp.accum == SPLAT_ACCUM_I32)
+            go(nd, std::integral_constant<int, SPLAT_ACCUM_I32>{});
+        else
+            go(nd, std::integral_constant<int, SPLAT_ACCUM_F32>{});
+    };
+    if (sp.n_delta == 2)
+        typed(std::integral_constant<int, 2>{});
+    else if (sp.n_delta == 1)
+        typed(std::integral_constant<int, 1>{});
+    else
+        typed(std::integral_constant<int, 0>{});
+}
+
 // continuum_light_map2! on the caller's AoS rays: final_evolution in place,
 // then the splat, one lane per diffuse ray walking all its planes as in
 // splat_kernel.  The block's diffuse rays are compacted through shared memory
@@ -313,9 +332,11 @@ cudaError_t launch_partition(splat_adray_t* rays, int64_t n, int64_t* counts, in
 // rays, 12 planes, 2 x 2 offsets: 311.7 -> 137.6 us (ncu, one GB300).  A block
 // of 128 for every 128 records, four at a time per SM: the whole frame of
 // those rays takes 632 us with blocks of 256 that go over the records in two
-// or more turns, and 617 so.
+// or more turns, and 617 so; 592 instead of 599 with a kernel per sample count
+// and map type.
 constexpr int kMapThreads = 128;
 
+template <int ND, int ACCUM>
 __global__ void __launch_bounds__(kMapThreads, 4) light_map_kernel(splat_adray_t* rays, int64_t n,
                                                                    const int32_t* __restrict__ hit_idx,
                                                                    const splat_ftri_t* __restrict__ tris,
@@ -327,6 +348,7 @@ __global__ void __launch_bounds__(kMapThreads, 4) light_map_kernel(splat_adray_t
     static_assert(sizeof(s_tile) >= sizeof(float) * (kPlanes + 1) * kMapThreads, "pool fits the tiles");
     const int lane = lane_id(), wid = threadIdx.x >> 5;
     AosTile& tile = s_tile[wid];
+    const DirectSink<SplatParams, ACCUM> sink{sp};
     const int planes = sp.n_lambda > 0 ? sp.n_lambda : 1;
     for (int64_t base = (int64_t)blockIdx.x * kMapThreads; base < n; base += (int64_t)gridDim.x * kMapThreads) {
         const int64_t wbase = base + 32 * wid, k = wbase + lane;
@@ -396,7 +418,7 @@ __global__ void __launch_bounds__(kMapThreads, 4) light_map_kernel(splat_adray_t
             s.y = q.f[26 * q.cap + p];
             const Tri T = load_tri(tris, __float_as_int(q.f[27 * q.cap + p]));
             const TriUV quv = tri_uv(T);
-            for (int il = 0; il < planes; ++il) (void)splat_ray_plane(sp, s, T, quv, il);
+            for (int il = 0; il < planes; ++il) (void)splat_ray_plane_n<ND>(sp, s, T, quv, il, sink);
         }
         __syncthreads();  // the tiles are free again
     }
@@ -406,7 +428,10 @@ cudaError_t launch_light_map(splat_adray_t* rays, int64_t n, const int32_t* hit_
                              int64_t n_tris, int32_t* err, const SplatParams& sp, int sm_count, cudaStream_t s) {
     if (n <= 0) return cudaSuccess;
     const int64_t b = std::min<int64_t>((n + kMapThreads - 1) / kMapThreads, (int64_t)sm_count * 64);
-    light_map_kernel<<<(int)b, kMapThreads, 0, s>>>(rays, n, hit_idx, tris, n_tris, err, sp);
+    by_form(sp, [&](auto nd, auto accum) {
+        light_map_kernel<decltype(nd)::value, decltype(accum)::value>
+            <<<(int)b, kMapThreads, 0, s>>>(rays, n, hit_idx, tris, n_tris, err, sp);
+    });
     ++g_launches;
     return cudaGetLastError();
 }
@@ -455,15 +480,6 @@ __global__ void __launch_bounds__(kSplatThreads, 5) splat_kernel(RaySoA q, Splat
         for (int il = 0; il < planes; ++il) done += splat_ray_plane_n<ND>(sp, r, T, quv, il, sink);
     }
     add_stats(st, 0, done);
-}
-
-template <int ND>
-static void launch_splat_nd(int grid, const RaySoA& q, const SplatRange& rg, const splat_ftri_t* tris,
-                            const SplatParams& sp, splat_trace_stats_t* stats, cudaStream_t s) {
-    if (sp.accum == SPLAT_ACCUM_I32)
-        splat_kernel<ND, SPLAT_ACCUM_I32><<<grid, kSplatThreads, 0, s>>>(q, rg, tris, sp, stats);
-    else
-        splat_kernel<ND, SPLAT_ACCUM_F32><<<grid, kSplatThreads, 0, s>>>(q, rg, tris, sp, stats);
 }
 
 // The same splat through the block's shared texel table: the block takes
@@ -516,12 +532,11 @@ cudaError_t launch_splat(const RaySoA& q, const SplatRange& rg, const splat_ftri
     if (b > lim) b = lim;
     if (agg)
         splat_agg_kernel<<<(int)b, threads, 0, s>>>(q, rg, tris, sp, stats);
-    else if (sp.n_delta == 2)
-        launch_splat_nd<2>((int)b, q, rg, tris, sp, stats, s);
-    else if (sp.n_delta == 1)
-        launch_splat_nd<1>((int)b, q, rg, tris, sp, stats, s);
     else
-        launch_splat_nd<0>((int)b, q, rg, tris, sp, stats, s);
+        by_form(sp, [&](auto nd, auto accum) {
+            splat_kernel<decltype(nd)::value, decltype(accum)::value>
+                <<<(int)b, threads, 0, s>>>(q, rg, tris, sp, stats);
+        });
     ++g_launches;
     return cudaGetLastError();
 }
