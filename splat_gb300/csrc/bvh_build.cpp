@@ -12,8 +12,11 @@
 // triangle.  Every triangle box is therefore padded by
 //   pad = pad_abs + pad_rel * |box diagonal|,
 //   pad_abs = 1e-4 * max(1, max |coordinate|),  pad_rel = 1e-3,
-// orders of magnitude above that rounding band, and traversal keeps every
-// node whose padded box the ray enters at or before the current best t.  The
+// orders of magnitude above that rounding band.  What grows with the distance
+// of a ray's origin, in the turned frame of the boxes above all, is no part of
+// it: the ray carries a slack of its own (slab_ray, hitcore.cuh).  Traversal
+// keeps every node whose box, so widened, the ray enters at or before the
+// current best t.  The
 // BVH hitter therefore tests every triangle whose test can succeed at
 // t <= best, and with the lexicographic (t, index) rule returns exactly the
 // brute-force result.  (Compiled with -ffp-contract=off like the device

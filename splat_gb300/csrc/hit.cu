@@ -780,7 +780,8 @@ __global__ void __launch_bounds__(kBvhThreads) hit_bvh_kernel(RaySrc src, BvhVie
         const int64_t k = src.perm ? (int64_t)src.perm[kk] : kk;
         const HitRay r = load_hit_ray<AOS>(src, k);
         const SlabRay sr = slab_ray(r, bvh.root4);
-        const float ix = sr.ix, iy = sr.iy, iz = sr.iz, oix = sr.oix, oiy = sr.oiy, oiz = sr.oiz;
+        // the near plane of an axis by the sign of the inverse direction, as in node4_slabs
+        const bool sx = sr.ix < 0.0f, sy = sr.iy < 0.0f, sz = sr.iz < 0.0f;
         float best = __int_as_float(0x7f800000);
         int32_t bi = 1;
         int sp = 0;
@@ -792,16 +793,14 @@ __global__ void __launch_bounds__(kBvhThreads) hit_bvh_kernel(RaySrc src, BvhVie
                 const float4 by = __ldg(&nd->y);
                 const float4 bz = __ldg(&nd->z);
                 const int4 c = __ldg(&nd->c);
-                const float a0 = fmaf(bx.x, ix, -oix), b0 = fmaf(bx.y, ix, -oix);
-                const float a1 = fmaf(by.x, iy, -oiy), b1 = fmaf(by.y, iy, -oiy);
-                const float a2 = fmaf(bz.x, iz, -oiz), b2 = fmaf(bz.y, iz, -oiz);
-                const float tmin0 = fmaxf(fmaxf(fminf(a0, b0), fminf(a1, b1)), fminf(a2, b2));
-                const float tmax0 = fminf(fminf(fmaxf(a0, b0), fmaxf(a1, b1)), fmaxf(a2, b2));
-                const float e0 = fmaf(bx.z, ix, -oix), f0 = fmaf(bx.w, ix, -oix);
-                const float e1 = fmaf(by.z, iy, -oiy), f1 = fmaf(by.w, iy, -oiy);
-                const float e2 = fmaf(bz.z, iz, -oiz), f2 = fmaf(bz.w, iz, -oiz);
-                const float tmin1 = fmaxf(fmaxf(fminf(e0, f0), fminf(e1, f1)), fminf(e2, f2));
-                const float tmax1 = fminf(fminf(fmaxf(e0, f0), fmaxf(e1, f1)), fmaxf(e2, f2));
+                const float a0 = fmaf(sx ? bx.y : bx.x, sr.ix, sr.nx), b0 = fmaf(sx ? bx.x : bx.y, sr.ix, sr.fx);
+                const float a1 = fmaf(sy ? by.y : by.x, sr.iy, sr.ny), b1 = fmaf(sy ? by.x : by.y, sr.iy, sr.fy);
+                const float a2 = fmaf(sz ? bz.y : bz.x, sr.iz, sr.nz), b2 = fmaf(sz ? bz.x : bz.y, sr.iz, sr.fz);
+                const float tmin0 = fmaxf(fmaxf(a0, a1), a2), tmax0 = fminf(fminf(b0, b1), b2);
+                const float e0 = fmaf(sx ? bx.w : bx.z, sr.ix, sr.nx), f0 = fmaf(sx ? bx.z : bx.w, sr.ix, sr.fx);
+                const float e1 = fmaf(sy ? by.w : by.z, sr.iy, sr.ny), f1 = fmaf(sy ? by.z : by.w, sr.iy, sr.fy);
+                const float e2 = fmaf(sz ? bz.w : bz.z, sr.iz, sr.nz), f2 = fmaf(sz ? bz.z : bz.w, sr.iz, sr.fz);
+                const float tmin1 = fmaxf(fmaxf(e0, e1), e2), tmax1 = fminf(fminf(f0, f1), f2);
                 const bool h0 = (tmin0 <= tmax0) & (tmax0 >= 0.0f) & (tmin0 <= best);
                 const bool h1 = (tmin1 <= tmax1) & (tmax1 >= 0.0f) & (tmin1 <= best);
                 if (h0 && h1) {

@@ -103,8 +103,8 @@ static_assert(sizeof(Bvh4Node) == 128, "Bvh4Node layout");
 // The frame a scene's BVH boxes are axis-aligned in, as rows of a matrix
 // applied to world positions and directions.  A linear map keeps the t of
 // every ray-box intersection, so traversal rotates each ray once (slab_ray)
-// and tests triangles in world space as before; only how tightly the boxes
-// fit changes.  The frame is the vector part of a unit quaternion with
+// and tests triangles in world space; only how tightly the boxes fit changes
+// (what turning a ray rounds is in its slack there).  The frame is the vector part of a unit quaternion with
 // w >= 0, kept as float bits in the four-wide root's meta.y, z, w; all zero
 // is the world frame.  Host build, refit and traversal derive the matrix
 // with the same binary32 operations.
