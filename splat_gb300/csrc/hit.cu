@@ -1078,8 +1078,11 @@ cudaError_t launch_hit_bvh4(const RaySrc& rays, int64_t cap, const Bvh4View& bvh
         prefer_l1(hit_bvh_kernel<false>);
         configured = true;
     }
+    RaySrc src = rays;
+    src.few = 0;  // set below where the group kernel is launched too
     if (g_tune[SPLAT_TUNE_COUNT_WORK]) {
-        launch_bvh4_form<true>(rays, cap, bvh, hit_idx, hit_t, err, sm_count, s);
+        // the counting forms take every ray: the group kernel does not count
+        launch_bvh4_form<true>(src, cap, bvh, hit_idx, hit_t, err, sm_count, s);
         ++g_launches;
         return cudaGetLastError();
     }
@@ -1088,7 +1091,6 @@ cudaError_t launch_hit_bvh4(const RaySrc& rays, int64_t cap, const Bvh4View& bvh
     // are launched and the count on the device picks the one that works.
     // Packet and refill forms that were asked for by their knobs stay.
     const bool groups = g_tune[SPLAT_TUNE_BVH_REFILL] == 0 && g_tune[SPLAT_TUNE_BVH_PACKET] <= 1;
-    RaySrc src = rays;
     src.few = groups && rays.few && rays.packet == 0 ? 1 : 0;
     const bool only = groups && cap <= kGroupRays;
     if (only || src.few) {
