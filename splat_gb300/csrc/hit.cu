@@ -445,12 +445,24 @@ cudaError_t launch_hit_brute_packed(const RaySrc& rays, int64_t cap, const TriHi
 // alone, so the box holds only for a plane normal that is the triangle's own
 // (an accepted point then lies in the triangle's plane) and for a triangle
 // that is no sliver (whose barycentrics' rounding moves points across its
-// edges): |n . edge| <= 2.5e-4 |n| |diagonal| and sin^2 of the corner at a
-// >= 1e-2.  With those the accepted points leave the triangle by less than
+// edges): |n . edge| <= 2.5e-4 |n| |edge| for both edges at a (measured by the
+// edge, not by the diagonal: a needle's short edge may be the normal's own
+// direction) and sin^2 of the corner at a >= 1e-2.  The normal then leans by
+// at most 5e-3, an accepted point is at most 2.5e-4 of an edge off the
+// triangle's plane, and all accepted points leave the triangle by less than
 // half the padding, 1e-3 of the diagonal plus 1e-4 max(1, largest
-// coordinate), as long as the ray starts within kNtrisReach of that scale.
-// A record without a normal (the sentinel) accepts nothing: an empty box.
+// coordinate), as long as the ray starts within kNtrisReach of that scale and
+// its direction is one that the box test keeps (plain_direction).  A record
+// without a normal (the sentinel) accepts nothing: an empty box.
 constexpr float kNtrisReach = 100.0f;
+// The box test raises components below 1e-30 to that (safe_inv), which moves a
+// point at distance t |d| by t 1e-30: nothing at 300 scales while |d| >= 1e-20.
+// From 1e30 on inverses are close to the subnormal ones.  A zero direction
+// accepts nothing, and idle lanes have one.
+__device__ __forceinline__ bool plain_direction(float dx, float dy, float dz) {
+    const float m = fmaxf(fmaxf(fabsf(dx), fabsf(dy)), fabsf(dz));
+    return (m >= 1.0e-20f && m <= 1.0e30f) || m == 0.0f;
+}
 __device__ __forceinline__ TriBox ntris_box(const TriHit& h, F3 a, F3 b, F3 c, float& scale) {
     const float inf = __int_as_float(0x7f800000);
     const F3 n = {h.n_nv.x, h.n_nv.y, h.n_nv.z}, e0 = {h.e0.x, h.e0.y, h.e0.z}, e1 = {h.e1.x, h.e1.y, h.e1.z};
@@ -460,8 +472,9 @@ __device__ __forceinline__ TriBox ntris_box(const TriHit& h, F3 a, F3 b, F3 c, f
     const float diag = sqrtf(dx * dx + dy * dy + dz * dz);
     scale = fmaxf(1.0f, fmaxf(fmaxf(fmaxf(fabsf(lx), fabsf(hx)), fmaxf(fabsf(ly), fabsf(hy))),
                               fmaxf(fabsf(lz), fabsf(hz))));
-    const float slack = (2.5e-4f * sqrtf(dot(n, n))) * diag;
-    const bool own = fabsf(dot(n, e0)) <= slack && fabsf(dot(n, e1)) <= slack && diag < inf;
+    const float lean = 2.5e-4f * sqrtf(dot(n, n));
+    const bool own =
+        fabsf(dot(n, e0)) <= lean * sqrtf(h.e0.w) && fabsf(dot(n, e1)) <= lean * sqrtf(h.e1.w) && diag < inf;
     const bool wide = h.inv.y * (h.e0.w * h.e1.w) <= 1.0e2f && h.inv.y > 0.0f;
     if (n.x == 0.0f && n.y == 0.0f && n.z == 0.0f)
         return TriBox{make_float4(inf, inf, inf, 0.f), make_float4(-inf, -inf, -inf, 0.f)};
@@ -531,7 +544,7 @@ __global__ void __launch_bounds__(kBruteThreads) hit_ntris_kernel(const splat_ad
     HitRay ray[kRPT];
     float best[kRPT], inv[kRPT][3], oinv[kRPT][3];
     int32_t bi[kRPT], bpos[kRPT];
-    float reach = 0.0f;  // largest |origin coordinate| over the warp
+    float reach = 0.0f;  // largest |origin coordinate| over the warp; infinite: some direction is not plain
 #pragma unroll
     for (int r = 0; r < kRPT; ++r) {
         const int64_t k = ray0 + (wid * kRPT + r) * 32 + lane;
@@ -545,6 +558,7 @@ __global__ void __launch_bounds__(kBruteThreads) hit_ntris_kernel(const splat_ad
         oinv[r][1] = ray[r].oy * inv[r][1];
         oinv[r][2] = ray[r].oz * inv[r][2];
         reach = fmaxf(reach, fmaxf(fmaxf(fabsf(ray[r].ox), fabsf(ray[r].oy)), fabsf(ray[r].oz)));
+        if (!plain_direction(ray[r].dx, ray[r].dy, ray[r].dz)) reach = inf;
     }
     reach = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(reach)));
     for (int64_t base = tb; base < te; base += kTile) {
@@ -622,7 +636,8 @@ __global__ void __launch_bounds__(kBruteThreads) hit_ntris_kernel(const splat_ad
         }
         if (lane == 0) box32[wid] = m;
         __syncthreads();
-        const bool all = !(reach <= kNtrisReach * s_scale);  // also a NaN reach
+        // (a NaN origin drops out of reach: its ray passes no triangle's test)
+        const bool all = !(reach <= kNtrisReach * s_scale);
 #pragma unroll
         for (int r = 0; r < kRPT; ++r) bpos[r] = -1;  // a best hit from an earlier tile wins ties
 #pragma unroll 1
