@@ -947,13 +947,14 @@ __global__ void __launch_bounds__(kBvhThreads) hit_bvh4_kernel(RaySrc src, Bvh4V
 template <bool AOS>
 __global__ void __launch_bounds__(kBvhThreads) hit_bvh4_group_kernel(RaySrc src, Bvh4View bvh,
                                                                      int32_t* __restrict__ hit_idx,
-                                                                     float* __restrict__ hit_t) {
+                                                                     float* __restrict__ hit_t, int32_t* err) {
     __shared__ int2 s_stack[kBvhThreads / 32][kGroupStackWarp];
     const int64_t n = src.d_count ? *src.d_count : src.n;
     if (n > kGroupRays) return;
     auto ray_of = [&](int64_t kk) { return src.perm ? (int64_t)src.perm[kk] : kk; };
     bvh4_groups(
-        n, src.fetch, s_stack[threadIdx.x >> 5], [&](int64_t kk) { return load_hit_ray<AOS>(src, ray_of(kk)); },
+        n, src.fetch, s_stack[threadIdx.x >> 5], err,
+        [&](int64_t kk) { return load_hit_ray<AOS>(src, ray_of(kk)); },
         [&](int64_t) { return bvh; },
         [&](int64_t kk, float best, int32_t bi) {
             const int64_t k = ray_of(kk);
@@ -1113,9 +1114,9 @@ cudaError_t launch_hit_bvh4(const RaySrc& rays, int64_t cap, const Bvh4View& bvh
         const int grid = resident_grid(reinterpret_cast<const void*>(hit_bvh4_group_kernel<false>), lanes, sm_count,
                                        kBvhThreads, 256);
         if (rays.aos)
-            hit_bvh4_group_kernel<true><<<grid, kBvhThreads, 0, s>>>(src, bvh, hit_idx, hit_t);
+            hit_bvh4_group_kernel<true><<<grid, kBvhThreads, 0, s>>>(src, bvh, hit_idx, hit_t, err);
         else
-            hit_bvh4_group_kernel<false><<<grid, kBvhThreads, 0, s>>>(src, bvh, hit_idx, hit_t);
+            hit_bvh4_group_kernel<false><<<grid, kBvhThreads, 0, s>>>(src, bvh, hit_idx, hit_t, err);
         ++g_launches;
         if (only) return cudaGetLastError();
     }

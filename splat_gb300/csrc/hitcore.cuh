@@ -512,8 +512,10 @@ __device__ __forceinline__ void bvh4_closest_packet(const HitRay& r, bool valid,
 // stack: kGroupStack<G> entries of shared memory per group.  A step takes no
 // more entries than the room above leaves space for (three net pushes each),
 // and with less than that it takes one, which needs at most kBvhStack more
-// entries (the builder's bound on three per level), so the stack cannot
-// overflow.
+// entries in a tree of the host builder (its bound on three per level).  A
+// tree rebuilt on the GPU has no such bound (30 levels of Morton bits, and
+// the logarithm of the triangles in one cell): a step whose children may not
+// fit passes them by and sets error bit 2, as the one-lane walk does.
 //
 // Measured on one GB300 (us a next_hit call, scattered rays; one lane a ray /
 // eight / thirty-two; a call's host work is about 15 us of each):
@@ -528,17 +530,29 @@ static_assert(kGroupStackWarp >= 4 * kGroupStack<8>, "one warp's stacks");
 constexpr int64_t kGroupWarpRays = 4096;
 constexpr int64_t kGroupRays = 16384;
 
+// Entries a step takes off a group's stack of sp, and, with sp left, whether
+// four children of each have room.
+template <int G>
+__host__ __device__ __forceinline__ int group_take(int sp) {
+    const int room = (kGroupStack<G> - kBvhStack - sp) / 3;
+    const int most = room > 1 ? room : 1;
+    return sp < G ? (sp < most ? sp : most) : (G < most ? G : most);
+}
+template <int G>
+__host__ __device__ __forceinline__ bool group_fits(int sp, int take) {
+    return sp + 4 * take <= kGroupStack<G>;
+}
+
 // One step of every group of the warp (all 32 lanes call; a group without
 // entries, sp = 0, idles).
 template <int G>
 __device__ __forceinline__ void bvh4_group_step(const HitRay& r, const SlabRay& sr, const Bvh4View& bvh, int2* stack,
-                                                int& sp, float& best, int32_t& bi) {
+                                                int32_t* err, int& sp, float& best, int32_t& bi) {
     const int lane = threadIdx.x & 31, gl = lane & (G - 1), g0 = lane & ~(G - 1);
     const unsigned gmask = G == 32 ? 0xffffffffu : ((1u << (G & 31)) - 1u) << g0;
     const unsigned below = (1u << lane) - 1u;
     __syncwarp();
-    const int room = (kGroupStack<G> - kBvhStack - sp) / 3;
-    const int take = min(min(sp, G), max(room, 1));
+    const int take = group_take<G>(sp);
     const bool mine = gl < take;
     sp -= take;
     int ref = 0;
@@ -558,8 +572,12 @@ __device__ __forceinline__ void bvh4_group_step(const HitRay& r, const SlabRay& 
         c = __ldg(&nd->c);
         float tmax[4];
         node4_slabs(nd, sr, tmin, tmax);
-    #pragma unroll
-        for (int i = 0; i < 4; ++i) h[i] = (tmin[i] <= tmax[i]) & (tmin[i] <= best);
+        if (!group_fits<G>(sp, take)) {
+            atomicOr(err, 2);
+        } else {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) h[i] = (tmin[i] <= tmax[i]) & (tmin[i] <= best);
+        }
     } else if (go) {
         const int enc = ~ref;
         const int first = enc >> 4;
@@ -607,8 +625,8 @@ __device__ __forceinline__ void bvh4_group_step(const HitRay& r, const SlabRay& 
 // load(k): ray k; view(k): the BVH it is traced in; store(k, t, index).
 // Groups take rays off the work counter, or stride statically without one.
 template <int G, class Load, class View, class Store>
-__device__ __forceinline__ void bvh4_group_loop(int64_t n, unsigned long long* fetch, int2* stack, const Load& load,
-                                                const View& view, const Store& store) {
+__device__ __forceinline__ void bvh4_group_loop(int64_t n, unsigned long long* fetch, int2* stack, int32_t* err,
+                                                const Load& load, const View& view, const Store& store) {
     static_assert(G == 8 || G == 32, "group size");
     const float kInf = __int_as_float(0x7f800000);
     const int lane = threadIdx.x & 31, gl = lane & (G - 1), g0 = lane & ~(G - 1);
@@ -658,7 +676,7 @@ __device__ __forceinline__ void bvh4_group_loop(int64_t n, unsigned long long* f
             if (!fetch) more = __any_sync(0xffffffffu, next < n);
         }
         if (!more && __all_sync(0xffffffffu, k < 0)) break;
-        bvh4_group_step<G>(r, sr, bvh, stack, sp, best, bi);
+        bvh4_group_step<G>(r, sr, bvh, stack, err, sp, best, bi);
     }
 }
 
@@ -666,25 +684,25 @@ __device__ __forceinline__ void bvh4_group_loop(int64_t n, unsigned long long* f
 // ray).  stack: the group's kGroupStack<G> entries.
 template <int G>
 __device__ __forceinline__ void bvh4_closest_group(const HitRay& r, bool live, const Bvh4View& bvh, int2* stack,
-                                                   float& best, int32_t& bi) {
+                                                   int32_t* err, float& best, int32_t& bi) {
     const SlabRay sr = slab_ray(r, bvh.nodes);
     best = __int_as_float(0x7f800000);
     bi = 1;
     int sp = live ? 1 : 0;
     __syncwarp();  // the stack's previous readers are done
     if (live && (threadIdx.x & (G - 1)) == 0) stack[0] = make_int2(0, 0);
-    while (__any_sync(0xffffffffu, sp > 0)) bvh4_group_step<G>(r, sr, bvh, stack, sp, best, bi);
+    while (__any_sync(0xffffffffu, sp > 0)) bvh4_group_step<G>(r, sr, bvh, stack, err, sp, best, bi);
 }
 
 // n <= kGroupRays rays by the group size that suits their number; stack: the
 // warp's kGroupStackWarp entries.
 template <class Load, class View, class Store>
-__device__ __forceinline__ void bvh4_groups(int64_t n, unsigned long long* fetch, int2* stack, const Load& load,
-                                            const View& view, const Store& store) {
+__device__ __forceinline__ void bvh4_groups(int64_t n, unsigned long long* fetch, int2* stack, int32_t* err,
+                                            const Load& load, const View& view, const Store& store) {
     if (n <= kGroupWarpRays)
-        bvh4_group_loop<32>(n, fetch, stack, load, view, store);
+        bvh4_group_loop<32>(n, fetch, stack, err, load, view, store);
     else
-        bvh4_group_loop<8>(n, fetch, stack + ((threadIdx.x & 31) >> 3) * kGroupStack<8>, load, view, store);
+        bvh4_group_loop<8>(n, fetch, stack + ((threadIdx.x & 31) >> 3) * kGroupStack<8>, err, load, view, store);
 }
 
 // Spread of a warp's rays, max over axes of (max - min) of a coordinate.

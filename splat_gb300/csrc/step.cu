@@ -60,7 +60,7 @@ __global__ void __launch_bounds__(kStepThreads) small_step_kernel(const __grid_c
         float t;
         int32_t i;
         if (A.nodes4)
-            bvh4_closest_group<kStepGroup>(hr, live, Bvh4View{A.nodes4, A.recs}, stack, t, i);
+            bvh4_closest_group<kStepGroup>(hr, live, Bvh4View{A.nodes4, A.recs}, stack, A.err, t, i);
         else
             brute_closest_group<kStepGroup>(hr, live, A.recs, A.boxes, A.n_recs, t, i);
         if (live) {
