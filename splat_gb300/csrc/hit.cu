@@ -385,19 +385,11 @@ static cudaError_t brute_launch(const RaySrc& rays, int64_t cap, const TriHit* r
     // triangles, 450 / 418 / 411 / 382 us a frame with 1 / 2 / 4 / 8), down to
     // one tile a block (1,024 rays, 322 triangles: 180 -> 129 us a frame)
     constexpr int64_t kScanSplit = 8;
-    int64_t splits =
-        (kScanSplit * sm_count * g_tune[SPLAT_TUNE_BRUTE_BLOCKS_PER_SM] + ray_blocks - 1) / ray_blocks;
     const int stall_tile = g_tune[SPLAT_TUNE_TEST_WAIT_STALL] - 1;
     const int64_t least = (stall_tile >= 0 ? 4 : 1) * (int64_t)tile;  // the stall wants a block's later tiles
-    const int64_t max_splits = (n_recs + least - 1) / least;
-    if (splits > max_splits) splits = max_splits;
-    if (splits < 1) splits = 1;
-    if (splits > 65535) splits = 65535;
-    if (tmp == nullptr) splits = 1;
-    int64_t per_split = (n_recs + splits - 1) / splits;
-    per_split = ((per_split + tile - 1) / tile) * tile;
-    splits = (n_recs + per_split - 1) / per_split;
-    if (splits < 1) splits = 1;
+    int64_t wanted = (kScanSplit * sm_count * g_tune[SPLAT_TUNE_BRUTE_BLOCKS_PER_SM] + ray_blocks - 1) / ray_blocks;
+    if (tmp == nullptr) wanted = 1;
+    const auto [splits, per_split] = split_records(n_recs, wanted, least, tile);
     const bool use_tmp = packed || splits > 1;
     if (use_tmp && !packed) {
         fill_u64_kernel<<<grid_for(cap, 256, sm_count, 8), 256, 0, s>>>((unsigned long long*)tmp, cap, rays.d_count,
@@ -697,15 +689,8 @@ cudaError_t launch_hit_brute_ntris(const splat_adray_t* rays, int64_t n_rays, co
     ++g_launches;
     const int64_t rays_per_block = (int64_t)kBruteThreads * kRPT;
     const int64_t ray_blocks = (n_rays + rays_per_block - 1) / rays_per_block;
-    int64_t splits = ((int64_t)sm_count * 4 + ray_blocks - 1) / ray_blocks;
-    const int64_t max_splits = (n_tris + kTile - 1) / kTile;
-    if (splits > max_splits) splits = max_splits;
-    if (splits < 1) splits = 1;
-    if (splits > 65535) splits = 65535;
-    int64_t per_split = (n_tris + splits - 1) / splits;
-    per_split = ((per_split + kTile - 1) / kTile) * kTile;
-    if (per_split < kTile) per_split = kTile;
-    splits = (n_tris + per_split - 1) / per_split;
+    const int64_t wanted = ((int64_t)sm_count * 4 + ray_blocks - 1) / ray_blocks;
+    const auto [splits, per_split] = split_records(n_tris, wanted, kTile, kTile);
     if (n_tris > 0) {
         dim3 grid((unsigned)ray_blocks, (unsigned)splits);
         hit_ntris_kernel<<<grid, kBruteThreads, 0, s>>>(rays, n_rays, ntris, n_tris, per_split,

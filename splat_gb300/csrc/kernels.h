@@ -170,6 +170,22 @@ __host__ __device__ inline BruteBoxes brute_boxes_of(const TriBox* all, int64_t 
     return {all, all + n_recs, all + n_recs + (n_recs + 7) / 8};
 }
 
+// n records as `splits` ranges of per_split (whole tiles), of at least `least`
+// records each where possible; wanted of them at most, one when there is none.
+struct RecordSplit {
+    int64_t splits, per_split;
+};
+__host__ __device__ inline RecordSplit split_records(int64_t n, int64_t wanted, int64_t least, int64_t tile) {
+    const int64_t most = (n + least - 1) / least;
+    int64_t s = wanted < most ? wanted : most;
+    s = s < 1 ? 1 : (s > 65535 ? 65535 : s);
+    int64_t per = (n + s - 1) / s;
+    per = (per + tile - 1) / tile * tile;
+    if (per < tile) per = tile;  // no records
+    s = (n + per - 1) / per;
+    return {s < 1 ? 1 : s, per};
+}
+
 // brute force over prepacked hit records (reference indices 2..T in any
 // order), each behind its padded box
 cudaError_t launch_hit_brute(const RaySrc& rays, int64_t cap, const TriHit* recs, const TriBox* boxes, int64_t n_recs,
