@@ -77,9 +77,11 @@ constexpr uint32_t kStallPolls = 64;
 // brute force, TMA-staged tiles
 // ---------------------------------------------------------------------------
 constexpr int kBruteThreads = 256;  // the n_tris drop-in kernel
-constexpr int kRPT = 2;
 constexpr int kTile = 256;  // records per tile of the n_tris drop-in kernel
-constexpr int kStages = 4;
+// Two stages of the ring: with four an SM holds half as many of the blocks of
+// 128 (2^20 scattered records on 1,282 triangles 1.14 against 1.11 ms, a frame
+// of 2^20 rays on 5,122 triangles 1.30 against 1.24 ms).
+constexpr int kStages = 2;
 
 // Every pair of a ray and a triangle is decided, but not one at a time: the
 // records are kept in a spatial order (the BVH's, or along a Morton curve
@@ -87,10 +89,15 @@ constexpr int kStages = 4;
 // consecutive records (box8, box32), and a box that no ray of a warp enters
 // at or before its best hit rules out its records as the record's own box
 // would.  The block first tests its rays against the merged boxes of a run of
-// kBruteRun tiles and lists the tiles some ray needs; only those are copied,
-// and in them a warp passes by the groups of 8 that none of its rays enters.
+// kBruteRun tiles and lists the tiles some ray needs; only those are copied.
+// In them every lane marks the groups of 8 its ray enters, then goes over its
+// own groups and, in each, over the records it may enter: lanes look at
+// different records.  (All lanes over every group that some lane enters is as
+// good while a warp's rays are neighbours, and slower than one box test a pair
+// where they are strangers: 2^20 scattered records on 1,282 triangles 1.37 ms
+// with one box test a pair, 1.50 ms so, 1.11 with the lanes' own groups.)
 // Ties take the smaller reference index, so the order does not show.  2^16
-// rays, 20,482 triangles, depth 3: 3.87 -> 0.38 ms a frame (one GB300;
+// rays, 20,482 triangles, depth 3: 3.87 -> 0.29 ms a frame (one GB300;
 // before, one box test a pair).  The merged boxes alone, over the
 // mesh's own order, gain nothing: a subdivided sphere lists neighbouring
 // triangles far apart.
@@ -103,9 +110,27 @@ constexpr int kBruteRun = 512;
 // others up (two rays a lane in blocks of 256: 515 against 450 us a frame of
 // 2^16 rays).
 constexpr int kScanThreads = 128;
-constexpr int kScanRPT = 1;
 
-template <int RPT, bool AOS, int TILE>
+// The groups of 8 that a tile of cnt records has, as bits.
+__device__ __forceinline__ uint32_t group_bits(int cnt) {
+    const int groups = (cnt + 7) / 8;
+    return groups >= 32 ? 0xffffffffu : (1u << groups) - 1u;
+}
+// Which of the 8 boxes of a group a lane's ray may enter, as bits.  Lanes look
+// at different groups, and where groups lie 256 bytes apart, equal boxes of all
+// of them are in the same banks: there a lane starts at box g of its group g.
+__device__ __forceinline__ uint32_t box_bits(const TriBox* box, int g, const float inv[3], const float oinv[3],
+                                             float best) {
+    uint32_t m = 0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int q = (i + g) & 7;
+        m |= (enters(box[q].lo, box[q].hi, inv, oinv, best) ? 1u : 0u) << q;
+    }
+    return m;
+}
+
+template <bool AOS, int TILE>
 __global__ void __launch_bounds__(kScanThreads) hit_brute_kernel(RaySrc src, const TriHit* __restrict__ recs,
                                                                   BruteBoxes boxes,
                                                                   int64_t n_recs, int64_t per_split,
@@ -128,7 +153,7 @@ __global__ void __launch_bounds__(kScanThreads) hit_brute_kernel(RaySrc src, con
     __shared__ __align__(8) uint64_t stall;
 
     const int64_t n = src.d_count ? *src.d_count : src.n;
-    const int64_t ray0 = (int64_t)blockIdx.x * kScanThreads * RPT;
+    const int64_t ray0 = (int64_t)blockIdx.x * kScanThreads;
     if (ray0 >= n) return;
     const int64_t tb = (int64_t)blockIdx.y * per_split;
     const int64_t te = min(n_recs, tb + per_split);
@@ -136,38 +161,21 @@ __global__ void __launch_bounds__(kScanThreads) hit_brute_kernel(RaySrc src, con
     const int n_tiles = (int)((te - tb + TILE - 1) / TILE);
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
 
-    // a warp's RPT x 32 rays are consecutive; a first bounce takes them in
-    // 8 x 4 tiles of the light grid, so that a block's rays are a patch of it
-    // (613 -> 515 us a frame of 2^16 rays: as columns of the grid its warps
-    // need different tiles and wait for one another at every one)
-    auto ray_at = [&](int r) {
-        const int64_t p = ray0 + (wid * RPT + r) * 32 + lane;
-        return src.tile_h > 0 && p < n && n < (int64_t(1) << 32)
-                   ? (int64_t)grid_tile_ray((uint32_t)p, (uint32_t)src.tile_h, (uint32_t)n)
-                   : p;
-    };
-    HitRay ray[RPT];
-    float best[RPT];
-    int32_t bi[RPT];
-    float inv[RPT][3], oinv[RPT][3];  // slab-test terms of the padded-box pre-test
-#pragma unroll
-    for (int r = 0; r < RPT; ++r) {
-        const int64_t k = ray_at(r);
-        if (k < n) {
-            ray[r] = load_hit_ray<AOS>(src, k);
-        } else {
-            ray[r] = HitRay{0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0};
-        }
-        // an idle lane's ray enters no box
-        best[r] = k < n ? __int_as_float(0x7f800000) : -__int_as_float(0x7f800000);
-        bi[r] = 1;
-        inv[r][0] = safe_inv(ray[r].dx);
-        inv[r][1] = safe_inv(ray[r].dy);
-        inv[r][2] = safe_inv(ray[r].dz);
-        oinv[r][0] = ray[r].ox * inv[r][0];
-        oinv[r][1] = ray[r].oy * inv[r][1];
-        oinv[r][2] = ray[r].oz * inv[r][2];
-    }
+    // a warp's rays are consecutive; a first bounce takes them in 8 x 4 tiles
+    // of the light grid, so that a block's rays are a patch of it (613 -> 515
+    // us a frame of 2^16 rays: as columns of the grid its warps need different
+    // tiles and wait for one another at every one)
+    const int64_t at = ray0 + threadIdx.x;
+    const int64_t k = src.tile_h > 0 && at < n && n < (int64_t(1) << 32)
+                          ? (int64_t)grid_tile_ray((uint32_t)at, (uint32_t)src.tile_h, (uint32_t)n)
+                          : at;
+    const HitRay ray = k < n ? load_hit_ray<AOS>(src, k) : HitRay{0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0};
+    // an idle lane's ray enters no box
+    float best = k < n ? __int_as_float(0x7f800000) : -__int_as_float(0x7f800000);
+    int32_t bi = 1;
+    // slab-test terms of the padded-box pre-test
+    const float inv[3] = {safe_inv(ray.dx), safe_inv(ray.dy), safe_inv(ray.dz)};
+    const float oinv[3] = {ray.ox * inv[0], ray.oy * inv[1], ray.oz * inv[2]};
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < kStages; ++s) mbar_init(&bars[s], 1);
@@ -207,8 +215,7 @@ __global__ void __launch_bounds__(kScanThreads) hit_brute_kernel(RaySrc src, con
                 for (int i = 0; i < TILE / 32; ++i) {
                     const TriBox* bx = boxes.box32 + min(b0 + i, last32);
                     const float4 lo = __ldg(&bx->lo), hi = __ldg(&bx->hi);
-#pragma unroll
-                    for (int r = 0; r < RPT; ++r) need |= enters(lo, hi, inv[r], oinv[r], best[r]);
+                    need |= enters(lo, hi, inv, oinv, best);
                 }
                 bits |= (__any_sync(0xffffffffu, need) ? 1u : 0u) << t;
             }
@@ -247,35 +254,27 @@ __global__ void __launch_bounds__(kScanThreads) hit_brute_kernel(RaySrc src, con
             const TriBox* btile = btiles + s * TILE;
             const TriBox* gtile = gtiles + s * (TILE / 8);
             if (s_need[wid][rel / 32] >> (rel & 31) & 1u) {
-                for (int g = 0; g * 8 < cnt; ++g) {
-                    bool in[RPT], some = false;
+                // each lane's groups of 8, then its records in them
+                uint32_t gm = 0;
 #pragma unroll
-                    for (int r = 0; r < RPT; ++r) {
-                        in[r] = enters(gtile[g].lo, gtile[g].hi, inv[r], oinv[r], best[r]);
-                        some |= in[r];
-                    }
-                    if (!__any_sync(0xffffffffu, some)) continue;
-                    const int j1 = min(cnt, g * 8 + 8);
-                    for (int q = g * 8; q < j1; ++q) {
-                        const float4 lo = btile[q].lo, hi = btile[q].hi;
-#pragma unroll
-                        for (int r = 0; r < RPT; ++r) {
-                            // the padded box first (the BVH leaves' test): a ray that misses it
-                            // cannot be accepted by the triangle's test
-                            if (!in[r] || !enters(lo, hi, inv[r], oinv[r], best[r])) continue;
-                            const float4 q0 = tile[q].n_nv;
-                            float num, den;
-                            if (!tri_candidate(q0, ray[r], best[r], num, den)) continue;
-                            const float4 q1 = tile[q].a_idx;
-                            const int32_t idx = __float_as_int(q1.w);
-                            bool inside;
-                            const float t =
-                                tri_t_from(num, den, q1, tile[q].e0, tile[q].e1, tile[q].inv, ray[r], inside);
-                            if (inside & (t > 0.0f) & (idx != ray[r].ig) &
-                                ((t < best[r]) | ((t == best[r]) & (idx < bi[r])))) {
-                                best[r] = t;
-                                bi[r] = idx;
-                            }
+                for (int g = 0; g < TILE / 8; ++g)
+                    gm |= (enters(gtile[g].lo, gtile[g].hi, inv, oinv, best) ? 1u : 0u) << g;
+                gm &= group_bits(cnt);
+                for (; gm; gm &= gm - 1) {
+                    const int g = __ffs(gm) - 1;
+                    uint32_t m = box_bits(btile + g * 8, g, inv, oinv, best);
+                    if (g * 8 + 8 > cnt) m &= (1u << (cnt - g * 8)) - 1u;
+                    for (; m; m &= m - 1) {
+                        const TriHit& h = tile[g * 8 + __ffs(m) - 1];
+                        float num, den;
+                        if (!tri_candidate(h.n_nv, ray, best, num, den)) continue;
+                        const float4 q1 = h.a_idx;
+                        const int32_t idx = __float_as_int(q1.w);
+                        bool inside;
+                        const float t = tri_t_from(num, den, q1, h.e0, h.e1, h.inv, ray, inside);
+                        if (inside & (t > 0.0f) & (idx != ray.ig) & ((t < best) | ((t == best) & (idx < bi)))) {
+                            best = t;
+                            bi = idx;
                         }
                     }
                 }
@@ -298,16 +297,12 @@ __global__ void __launch_bounds__(kScanThreads) hit_brute_kernel(RaySrc src, con
         return;
     }
 
-#pragma unroll
-    for (int r = 0; r < RPT; ++r) {
-        const int64_t k = ray_at(r);
-        if (k >= n) continue;
-        if (tmp) {
-            if (bi[r] != 1) atomicMin(tmp + k, (unsigned long long)pack_argmin(best[r], (uint32_t)bi[r]));
-        } else {
-            hit_idx[k] = bi[r];
-            if (hit_t) hit_t[k] = best[r];
-        }
+    if (k >= n) return;
+    if (tmp) {
+        if (bi != 1) atomicMin(tmp + k, (unsigned long long)pack_argmin(best, (uint32_t)bi));
+    } else {
+        hit_idx[k] = bi;
+        if (hit_t) hit_t[k] = best;
     }
 }
 
@@ -358,16 +353,16 @@ static void launch_brute_tiles(dim3 grid, cudaStream_t s, const RaySrc& rays, co
     const size_t smem = (size_t)kStages * (TILE * (sizeof(TriHit) + sizeof(TriBox)) + TILE / 8 * sizeof(TriBox));
     static bool configured = false;  // rings above 48 KB need the opt-in
     if (!configured) {
-        cudaFuncSetAttribute(hit_brute_kernel<kScanRPT, true, TILE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        cudaFuncSetAttribute(hit_brute_kernel<kScanRPT, false, TILE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        cudaFuncSetAttribute(hit_brute_kernel<true, TILE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaFuncSetAttribute(hit_brute_kernel<false, TILE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)smem);
         configured = true;
     }
     if (rays.aos)
-        hit_brute_kernel<kScanRPT, true, TILE><<<grid, kScanThreads, smem, s>>>(rays, recs, boxes, n_recs, per_split,
+        hit_brute_kernel<true, TILE><<<grid, kScanThreads, smem, s>>>(rays, recs, boxes, n_recs, per_split,
                                                                              hit_idx, hit_t, tmp, err, stall_tile);
     else
-        hit_brute_kernel<kScanRPT, false, TILE><<<grid, kScanThreads, smem, s>>>(rays, recs, boxes, n_recs, per_split,
+        hit_brute_kernel<false, TILE><<<grid, kScanThreads, smem, s>>>(rays, recs, boxes, n_recs, per_split,
                                                                               hit_idx, hit_t, tmp, err, stall_tile);
 }
 
@@ -378,7 +373,7 @@ static cudaError_t brute_launch(const RaySrc& rays, int64_t cap, const TriHit* r
     if (cap <= 0) return cudaSuccess;
     const BruteBoxes boxes = brute_boxes_of(all_boxes, n_recs);
     const int tile = g_tune[SPLAT_TUNE_BRUTE_TILE].load();
-    const int64_t rays_per_block = (int64_t)kScanThreads * kScanRPT;
+    const int64_t rays_per_block = kScanThreads;
     const int64_t ray_blocks = (cap + rays_per_block - 1) / rays_per_block;
     // split the triangle range so the grid covers the GPU several times over
     // (kScanSplit blocks of 128 for each of the knob's: 2^16 rays, 20,482
@@ -507,12 +502,23 @@ __device__ __forceinline__ uint32_t spread8(uint32_t x) {  // 8 bits, two zeros 
 
 // A tile of 256 of the caller's records is packed, given boxes (ntris_box) and
 // put along a Morton curve of its own box, so that boxes merged over 8 and 32
-// of them are small whatever order the array has; a warp passes by those none
-// of its rays enters (a warp with a ray too far out for the boxes tests every
-// triangle).  Equal distances take the earlier record, as over the array's
-// order: pos is the record's place in its tile.  40,000 rays, 5,123
-// triangles: 583 -> 127 us (ncu, one GB300; a division and the full test for
-// every pair before; boxes in the array's order 268).
+// of them are small whatever order the array has; a warp passes by those over
+// 32 that none of its rays enters, and every lane goes over the groups of 8 of
+// its own ray as in hit_brute_kernel (a warp with a ray too far out for the
+// boxes tests every triangle).  Equal distances take the earlier record, as
+// over the array's order: pos is the record's place in its tile.  Scattered /
+// gridded rays, us a call (a division and the full test for every pair; all
+// lanes over every group that some lane enters, two rays a lane; now):
+//   322 triangles, 2^16 rays    71 / 76         106 / 56      59 / 46
+//   1,282, 2^16                 206             190           112
+//   5,122, 300,000              3,026 / 3,374   2,170 / 634   1,175 / 663
+// Boxes of 8 records; the padding puts equal ones of different groups into
+// different banks.
+struct TriBox8 {
+    TriBox b[8];
+    float4 pad;
+};
+
 __global__ void __launch_bounds__(kBruteThreads) hit_ntris_kernel(const splat_adray_t* __restrict__ rays,
                                                                    int64_t n_rays, const splat_ntri_t* __restrict__ nt,
                                                                    int64_t n_tris, int64_t per_split,
@@ -520,7 +526,8 @@ __global__ void __launch_bounds__(kBruteThreads) hit_ntris_kernel(const splat_ad
     static_assert(kTile == kBruteThreads && kTile == 256, "a record a thread");
     constexpr int kWarps = kBruteThreads / 32;
     __shared__ TriHit tile[kTile];  // inv.z: pos
-    __shared__ TriBox box[kTile], box8[kTile / 8], box32[kTile / 32];
+    __shared__ __align__(16) TriBox8 box[kTile / 8];
+    __shared__ TriBox box8[kTile / 8], box32[kTile / 32];
     __shared__ float s_ext[kWarps][7];
     __shared__ uint32_t s_key[kTile];
     __shared__ float s_scale;
@@ -528,30 +535,19 @@ __global__ void __launch_bounds__(kBruteThreads) hit_ntris_kernel(const splat_ad
     RaySrc src{};
     src.aos = rays;
     src.n = n_rays;
-    const int64_t ray0 = (int64_t)blockIdx.x * kBruteThreads * kRPT;
     const int64_t tb = (int64_t)blockIdx.y * per_split;
     const int64_t te = min(n_tris, tb + per_split);
     if (tb >= te) return;
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-    HitRay ray[kRPT];
-    float best[kRPT], inv[kRPT][3], oinv[kRPT][3];
-    int32_t bi[kRPT], bpos[kRPT];
-    float reach = 0.0f;  // largest |origin coordinate| over the warp; infinite: some direction is not plain
-#pragma unroll
-    for (int r = 0; r < kRPT; ++r) {
-        const int64_t k = ray0 + (wid * kRPT + r) * 32 + lane;
-        ray[r] = k < n_rays ? load_hit_ray<true>(src, k) : HitRay{0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0};
-        best[r] = k < n_rays ? inf : -inf;  // an idle lane's ray enters no box
-        bi[r] = 1;
-        inv[r][0] = safe_inv(ray[r].dx);
-        inv[r][1] = safe_inv(ray[r].dy);
-        inv[r][2] = safe_inv(ray[r].dz);
-        oinv[r][0] = ray[r].ox * inv[r][0];
-        oinv[r][1] = ray[r].oy * inv[r][1];
-        oinv[r][2] = ray[r].oz * inv[r][2];
-        reach = fmaxf(reach, fmaxf(fmaxf(fabsf(ray[r].ox), fabsf(ray[r].oy)), fabsf(ray[r].oz)));
-        if (!plain_direction(ray[r].dx, ray[r].dy, ray[r].dz)) reach = inf;
-    }
+    const int64_t k = (int64_t)blockIdx.x * kBruteThreads + tid;
+    const HitRay ray = k < n_rays ? load_hit_ray<true>(src, k) : HitRay{0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0};
+    float best = k < n_rays ? inf : -inf;  // an idle lane's ray enters no box
+    int32_t bi = 1;
+    const float inv[3] = {safe_inv(ray.dx), safe_inv(ray.dy), safe_inv(ray.dz)};
+    const float oinv[3] = {ray.ox * inv[0], ray.oy * inv[1], ray.oz * inv[2]};
+    // largest |origin coordinate| over the warp; infinite: some direction is not plain
+    float reach = fmaxf(fmaxf(fabsf(ray.ox), fabsf(ray.oy)), fabsf(ray.oz));
+    if (!plain_direction(ray.dx, ray.dy, ray.dz)) reach = inf;
     reach = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(reach)));
     for (int64_t base = tb; base < te; base += kTile) {
         const int cnt = (int)min((int64_t)kTile, te - base);
@@ -614,9 +610,9 @@ __global__ void __launch_bounds__(kBruteThreads) hit_ntris_kernel(const splat_ad
         __syncthreads();
         const int slot = (int)s_key[tid];
         if (tid < cnt) tile[slot] = h;
-        box[slot] = m;
+        box[slot >> 3].b[slot & 7] = m;
         __syncthreads();
-        m = box[tid];
+        m = box[tid >> 3].b[tid & 7];
         for (int o = 1; o < 32; o <<= 1) {
             m.lo.x = fminf(m.lo.x, __shfl_xor_sync(0xffffffffu, m.lo.x, o));
             m.lo.y = fminf(m.lo.y, __shfl_xor_sync(0xffffffffu, m.lo.y, o));
@@ -630,55 +626,85 @@ __global__ void __launch_bounds__(kBruteThreads) hit_ntris_kernel(const splat_ad
         __syncthreads();
         // (a NaN origin drops out of reach: its ray passes no triangle's test)
         const bool all = !(reach <= kNtrisReach * s_scale);
-#pragma unroll
-        for (int r = 0; r < kRPT; ++r) bpos[r] = -1;  // a best hit from an earlier tile wins ties
+        int32_t bpos = -1;  // a best hit from an earlier tile wins ties
+        uint32_t gm = 0;
 #pragma unroll 1
         for (int part = 0; part * 32 < cnt; ++part) {
-            bool some = all;
-#pragma unroll
-            for (int r = 0; r < kRPT; ++r) some |= enters(box32[part].lo, box32[part].hi, inv[r], oinv[r], best[r]);
+            const bool some = all || enters(box32[part].lo, box32[part].hi, inv, oinv, best);
             if (!__any_sync(0xffffffffu, some)) continue;
+#pragma unroll
+            for (int g = 0; g < 4; ++g) {
+                const TriBox& b = box8[part * 4 + g];
+                gm |= (all || enters(b.lo, b.hi, inv, oinv, best) ? 1u : 0u) << (part * 4 + g);
+            }
+        }
 #pragma unroll 1
-            for (int g = part * 4; g < part * 4 + 4 && g * 8 < cnt; ++g) {
-                bool in[kRPT];
-                some = false;
-#pragma unroll
-                for (int r = 0; r < kRPT; ++r) {
-                    in[r] = all || enters(box8[g].lo, box8[g].hi, inv[r], oinv[r], best[r]);
-                    some |= in[r];
-                }
-                if (!__any_sync(0xffffffffu, some)) continue;
-                const int j1 = min(cnt, g * 8 + 8);
-                for (int j = g * 8; j < j1; ++j) {
-                    const float4 q0 = tile[j].n_nv;
-#pragma unroll
-                    for (int r = 0; r < kRPT; ++r) {
-                        if (!in[r] || !(all || enters(box[j].lo, box[j].hi, inv[r], oinv[r], best[r]))) continue;
-                        float num, den;
-                        if (!tri_candidate(q0, ray[r], best[r], num, den)) continue;
-                        const float4 q1 = tile[j].a_idx, q4 = tile[j].inv;
-                        const int32_t idx = __float_as_int(q1.w), pos = __float_as_int(q4.z);
-                        bool inside;
-                        const float t = tri_t_from(num, den, q1, tile[j].e0, tile[j].e1, q4, ray[r], inside);
-                        // next_hit_kernel6 (src/hitters.jl:183) has no i != 1 test: the
-                        // sentinel's t is NaN and fails t > 0.
-                        if (inside & (t > 0.0f) & (idx != ray[r].ig) &
-                            ((t < best[r]) | ((t == best[r]) & (pos < bpos[r])))) {
-                            best[r] = t;
-                            bi[r] = idx;
-                            bpos[r] = pos;
-                        }
-                    }
+        for (gm &= group_bits(cnt); gm; gm &= gm - 1) {
+            const int g = __ffs(gm) - 1;
+            uint32_t m = all ? 0xffu : box_bits(box[g].b, 0, inv, oinv, best);
+            if (g * 8 + 8 > cnt) m &= (1u << (cnt - g * 8)) - 1u;
+#pragma unroll 1
+            for (; m; m &= m - 1) {
+                const TriHit& h = tile[g * 8 + __ffs(m) - 1];
+                float num, den;
+                if (!tri_candidate(h.n_nv, ray, best, num, den)) continue;
+                const float4 q1 = h.a_idx, q4 = h.inv;
+                const int32_t idx = __float_as_int(q1.w), pos = __float_as_int(q4.z);
+                bool inside;
+                const float t = tri_t_from(num, den, q1, h.e0, h.e1, q4, ray, inside);
+                // next_hit_kernel6 (src/hitters.jl:183) has no i != 1 test: the
+                // sentinel's t is NaN and fails t > 0.
+                if (inside & (t > 0.0f) & (idx != ray.ig) & ((t < best) | ((t == best) & (pos < bpos)))) {
+                    best = t;
+                    bi = idx;
+                    bpos = pos;
                 }
             }
         }
         __syncthreads();
     }
-#pragma unroll
-    for (int r = 0; r < kRPT; ++r) {
-        const int64_t k = ray0 + (wid * kRPT + r) * 32 + lane;
-        if (k < n_rays && bi[r] != 1) atomicMin(tmp + k, (unsigned long long)pack_argmin(best[r], (uint32_t)bi[r]));
+    if (k < n_rays && bi != 1) atomicMin(tmp + k, (unsigned long long)pack_argmin(best, (uint32_t)bi));
+}
+
+// Up to kNtrisDirect records: every one against every ray, for the boxes and
+// their order take longer to make than they save.  us a call, boxes / none:
+//   42 triangles    2^20 rays 150 / 124   300,000 of a grid 58 / 58
+//   82              246 / 209             70 / 77
+//   128             244 / 309             73 / 107
+constexpr int kNtrisDirect = 96;
+__global__ void __launch_bounds__(kBruteThreads) hit_ntris_direct_kernel(const splat_adray_t* __restrict__ rays,
+                                                                          int64_t n_rays,
+                                                                          const splat_ntri_t* __restrict__ nt,
+                                                                          int n_tris,
+                                                                          unsigned long long* __restrict__ tmp) {
+    __shared__ TriHit tile[kNtrisDirect];
+    RaySrc src{};
+    src.aos = rays;
+    src.n = n_rays;
+    const int tid = threadIdx.x;
+    const int64_t k = (int64_t)blockIdx.x * kBruteThreads + tid;
+    const HitRay ray = k < n_rays ? load_hit_ray<true>(src, k) : HitRay{0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0};
+    float best = __int_as_float(0x7f800000);
+    int32_t bi = 1;
+    if (tid < n_tris) {
+        const splat_ntri_t& q = nt[tid];
+        tile[tid] = pack_one(q.idx, f3(q.v[0]), f3(q.v[1]), f3(q.v[2]), f3(q.v[3]));
     }
+    __syncthreads();
+#pragma unroll 2
+    for (int j = 0; j < n_tris; ++j) {
+        float num, den;
+        if (!tri_candidate(tile[j].n_nv, ray, best, num, den)) continue;
+        const float4 q1 = tile[j].a_idx;
+        const int32_t idx = __float_as_int(q1.w);
+        bool inside;
+        const float t = tri_t_from(num, den, q1, tile[j].e0, tile[j].e1, tile[j].inv, ray, inside);
+        if (inside & (t > 0.0f) & (idx != ray.ig) & (t < best)) {
+            best = t;
+            bi = idx;
+        }
+    }
+    if (k < n_rays && bi != 1) atomicMin(tmp + k, (unsigned long long)pack_argmin(best, (uint32_t)bi));
 }
 
 cudaError_t launch_hit_brute_ntris(const splat_adray_t* rays, int64_t n_rays, const splat_ntri_t* ntris,
@@ -687,18 +713,22 @@ cudaError_t launch_hit_brute_ntris(const splat_adray_t* rays, int64_t n_rays, co
     fill_u64_kernel<<<grid_for(n_rays, 256, sm_count, 8), 256, 0, s>>>((unsigned long long*)tmp, n_rays, nullptr,
                                                                        (unsigned long long)kNoHit);
     ++g_launches;
-    const int64_t rays_per_block = (int64_t)kBruteThreads * kRPT;
+    const int64_t rays_per_block = kBruteThreads;
     const int64_t ray_blocks = (n_rays + rays_per_block - 1) / rays_per_block;
     const int64_t wanted = ((int64_t)sm_count * 4 + ray_blocks - 1) / ray_blocks;
     const auto [splits, per_split] = split_records(n_tris, wanted, kTile, kTile);
-    if (n_tris > 0) {
+    if (n_tris > kNtrisDirect) {
         dim3 grid((unsigned)ray_blocks, (unsigned)splits);
         hit_ntris_kernel<<<grid, kBruteThreads, 0, s>>>(rays, n_rays, ntris, n_tris, per_split,
                                                          (unsigned long long*)tmp);
         ++g_launches;
-        cudaError_t e = cudaGetLastError();
-        if (e != cudaSuccess) return e;
+    } else if (n_tris > 0) {
+        hit_ntris_direct_kernel<<<(unsigned)ray_blocks, kBruteThreads, 0, s>>>(rays, n_rays, ntris, (int)n_tris,
+                                                                               (unsigned long long*)tmp);
+        ++g_launches;
     }
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
     return launch_unpack_hits(tmp, n_rays, nullptr, hit_idx, nullptr, s);
 }
 
