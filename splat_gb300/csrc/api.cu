@@ -798,15 +798,19 @@ static int64_t grid_rays(const splat_trace_params_t* P) {
 // the default forms (a knob that asks for a form of the separate kernels gets
 // them).  Measured on one GB300, us a step, separate launches -> one, at
 // 1,024 / 4,096 / 8,100 / 16,384 / 32,761 rays (depth 3, 4 planes, 2 x 2):
-//   sphere, 322 triangles, brute force   125/131/132/133/141 -> 60/64/73/114/193
 //   displaced sphere, 81,922, BVH        111/129/146/154/444 -> 77/84/99/149/249
 //   sponge, 96,012, BVH                  122/141/175/192/247 -> 85/98/140/210/371
-//   sphere, 20,482, brute force          144/193/232/289/320 -> 163/169/188/281/452
-// and 5,472 rays on a sponge of 4,813 by brute force, depth 6: 518 -> 631 (its
-// boxes overlap, and a group meets them in no particular order).
+// and by brute force at 1,024 / 4,096 / 8,100 / 12,288 rays (1 x 1 samples):
+//   sphere, 82 triangles                 89/90/92/90 -> 54/52/62/81
+//   sphere, 322                          91/89/92/91 -> 67/63/74/101
+//   displaced sphere, 702                88/89/90/91 -> 77/72/79/108
+//   900 small ones, scattered            84/86/87/91 -> 106/88/90/113
+//   900 as large as the scene            107/114/136/154 -> 214/179/241/297
+// (a group meets overlapping boxes in no particular order).
 static bool small_step(const splat_scene_t* scene, const splat_trace_params_t* P, int64_t cnt) {
-    return cnt <= kSmallStepRays && (P->hitter == SPLAT_HITTER_BVH || P->hitter == SPLAT_HITTER_BRUTE) &&
-           (P->hitter == SPLAT_HITTER_BVH || scene->n_recs <= kSmallStepBruteRecs) &&
+    const bool bvh = P->hitter == SPLAT_HITTER_BVH;
+    return (bvh || P->hitter == SPLAT_HITTER_BRUTE) && cnt <= kSmallStepRays &&
+           (bvh || scene->n_recs <= (cnt <= kSmallStepBruteRays ? kSmallStepBruteRecs : kSmallStepFewRecs)) &&
            g_tune[SPLAT_TUNE_BVH_PACKET] <= 1 &&
            g_tune[SPLAT_TUNE_BVH_REFILL] == 0 && g_tune[SPLAT_TUNE_RAY_ORDER] == 0 &&
            g_tune[SPLAT_TUNE_SPLAT_AGGREGATE] == 0 && g_tune[SPLAT_TUNE_COUNT_WORK] == 0 &&

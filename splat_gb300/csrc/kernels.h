@@ -387,7 +387,9 @@ cudaError_t launch_map_to_array(const int32_t* map, int64_t w, int64_t h, int64_
 // nodes4 null is the brute-force hitter; ea gives scene, material and draws
 // (its queues are unused).  stats accumulate, as the last splat leaves them.
 constexpr int64_t kSmallStepRays = 12288;
-constexpr int64_t kSmallStepBruteRecs = 1024;
+// by brute force: of at most kSmallStepBruteRecs records, above
+// kSmallStepBruteRays rays of kSmallStepFewRecs
+constexpr int64_t kSmallStepBruteRays = 8192, kSmallStepBruteRecs = 1024, kSmallStepFewRecs = 128;
 cudaError_t launch_small_step(const GenParams& gen, int64_t n, const Bvh4Node* nodes4, const TriHit* recs,
                               const TriBox* boxes, int64_t n_recs, const EvolveArgs& ea, int32_t depth,
                               const SplatParams& sp, splat_trace_stats_t* stats, cudaStream_t s);
