@@ -181,6 +181,12 @@ cudaError_t launch_evolve_plugin(const EvolveArgs& a, int64_t cap, int sm_count,
     return launch_evolve_mode<0>(a, cap, sm_count, s);
 }
 
+// A warp with at most this many records to change reads and writes those in
+// place: moving all 32 for them is wasted traffic.  2^20 records, one evolve,
+// us: 3 % active 118 all moved, 97 so; 10 % 130, 107; 20 % 129, 112; a third,
+// the line, 129, 136.
+constexpr int kSparseRecords = 12;
+
 // evolve_ray broadcast (src/tracer.jl:181-201: `rays .= evolve_ray.(rays,
 // hit_idx, tri_view, rndm, first_diffuse)`) on the caller's AoS rays: every
 // ACTIVE ray evolves in place with its hit index and its Fresnel draw
@@ -199,10 +205,12 @@ __global__ void __launch_bounds__(kEvolveThreads) evolve_aos_kernel(splat_adray_
         const int64_t k = base + lane;
         // the status first: a warp of retired rays moves nothing
         const bool act = k < n && rays[k].status == kStatusActive;
-        if (!__any_sync(kFull, act)) continue;
-        aos_tile_load(tile, rays, base, n);
+        const unsigned m = __ballot_sync(kFull, act);
+        if (m == 0) continue;
+        const bool dense = __popc(m) > kSparseRecords;
+        if (dense) aos_tile_load(tile, rays, base, n);
         if (act) {
-            splat_adray_t& a = aos_tile_ray(tile);
+            splat_adray_t& a = dense ? aos_tile_ray(tile) : rays[k];
             const RayState r = ray_from_aos(a);
             const EvolveView v{A.tris, A.n_tris, A.err, A.first_diffuse, A.material, A.seed, A.bounce,
                                rndm ? rndm[k] : A.force_rand, quirks, false};
@@ -213,7 +221,7 @@ __global__ void __launch_bounds__(kEvolveThreads) evolve_aos_kernel(splat_adray_
             else if (fate == kFateDiffuse) a.status = (uint8_t)kStatusDiffuse;
             else if (fate == kFateInfinity) a.status = (uint8_t)kStatusInfinity;
         }
-        aos_tile_store(tile, rays, base, n);
+        if (dense) aos_tile_store(tile, rays, base, n);
     }
 }
 
@@ -333,7 +341,10 @@ static void by_form(const SplatParams& sp, const Go& go) {
 // of 128 for every 128 records, four at a time per SM: the whole frame of
 // those rays takes 632 us with blocks of 256 that go over the records in two
 // or more turns, and 617 so; 592 instead of 599 with a kernel per sample count
-// and map type.
+// and map type.  A block with few diffuse rays spreads each ray's planes over
+// 2, 4, ... threads (2^20 records, 8 planes, 2 x 2: 1 % diffuse 166 -> 67 us,
+// 10 % 216 -> 89, 35 % 228 -> 157), and a warp with few of them leaves the
+// other records where they are (kSparseRecords).
 constexpr int kMapThreads = 128;
 
 template <int ND, int ACCUM>
@@ -356,12 +367,14 @@ __global__ void __launch_bounds__(kMapThreads, 4) light_map_kernel(splat_adray_t
         RayState o;
         int32_t ih = 1;
         const bool want = k < n && rays[k].status == kStatusDiffuse;
-        if (__any_sync(kFull, want)) {
-            aos_tile_load(tile, rays, wbase, n);
+        const unsigned wm = __ballot_sync(kFull, want);
+        if (wm) {
+            const bool dense = __popc(wm) > kSparseRecords;
+            if (dense) aos_tile_load(tile, rays, wbase, n);
             if (want) {
                 const int32_t i = hit_idx[k];
                 if (i >= 1 && i <= n_tris) {
-                    splat_adray_t& a = aos_tile_ray(tile);
+                    splat_adray_t& a = dense ? aos_tile_ray(tile) : rays[k];
                     const RayState r = ray_from_aos(a);
                     const Tri T = load_tri(tris, i);
                     HitDerivs h;
@@ -373,7 +386,7 @@ __global__ void __launch_bounds__(kMapThreads, 4) light_map_kernel(splat_adray_t
                     atomicOr(err, 16);
                 }
             }
-            aos_tile_store(tile, rays, wbase, n);
+            if (dense) aos_tile_store(tile, rays, wbase, n);
         }
         const unsigned db = __ballot_sync(kFull, dif);
         if (lane == 0) s_cnt[wid] = __popc(db);
@@ -402,8 +415,11 @@ __global__ void __launch_bounds__(kMapThreads, 4) light_map_kernel(splat_adray_t
             q.f[27 * q.cap + p] = __int_as_float(ih);
         }
         __syncthreads();
-        if ((int)threadIdx.x < total) {
-            const int p = threadIdx.x;
+        // few rays: 2, 4, ... threads a ray, each with every 2nd, 4th, ... plane
+        int spread = 0;
+        while (total << (spread + 1) <= kMapThreads && 1 << spread < planes) ++spread;
+        const int p = threadIdx.x >> spread;
+        if (p < total) {
             RayState s;
             s.pos = ld3(q.f, q.cap, 0, p);
             s.dir = ld3(q.f, q.cap, 3, p);
@@ -418,7 +434,8 @@ __global__ void __launch_bounds__(kMapThreads, 4) light_map_kernel(splat_adray_t
             s.y = q.f[26 * q.cap + p];
             const Tri T = load_tri(tris, __float_as_int(q.f[27 * q.cap + p]));
             const TriUV quv = tri_uv(T);
-            for (int il = 0; il < planes; ++il) (void)splat_ray_plane_n<ND>(sp, s, T, quv, il, sink);
+            for (int il = threadIdx.x & ((1 << spread) - 1); il < planes; il += 1 << spread)
+                (void)splat_ray_plane_n<ND>(sp, s, T, quv, il, sink);
         }
         __syncthreads();  // the tiles are free again
     }
