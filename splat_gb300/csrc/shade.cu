@@ -12,6 +12,7 @@
 // hardware linear filtering, clamped addressing and unnormalised coordinates,
 // sampled at (u, v, plane) - 0.5 (Julia's 1-based texel centres).
 #include <cmath>
+#include <type_traits>
 
 #include "optics.cuh"
 
@@ -31,13 +32,16 @@ namespace splat {
 //
 // Double arithmetic is what bounds these kernels (about two lanes a clock and
 // SM).  Everything of one row or one column is the same for the whole line of
-// the grid: a block takes a tile of kCamRows x kCamCols rays, computes its
+// the grid: a block takes a tile of ROWS x kCamTile / ROWS rays, computes its
 // rows' and columns' terms once into shared memory, and each ray is left with
 // one square root, one division and 40 adds, products and roundings, where it
 // had five divisions and twice as many: 230,400 rays 56 -> 35 us, 57,960
 // records 23 -> 13.5 us.
-constexpr int kCamRows = 32;  // a warp's lanes: consecutive rays
-constexpr int kCamCols = 16;
+// ROWS: 32, a warp's lanes being consecutive rays, for grids of more than 16
+// rows; lower ones would leave lanes idle and take 8 rows, or one.  us for
+// records of 1 x 100,000, 5 x 30,000, 9 x 20,000, 16 x 10,000 rays: without
+// tiles 41, 49, 57, 61; by 32 rows 353, 120, 87, 55; by these 37, 47, 58, 42.
+constexpr int kCamTile = 512;
 constexpr int kCamThreads = 256;
 
 struct CamRow {
@@ -50,32 +54,34 @@ struct CamCol {
 // Camera rays of tile t (0-based ray g = x + h y, x and y 1-based in the
 // formulas above); their jitter dv = three uniforms of Philox(seed) at
 // (g, 0, 2, 0).  put(g, ray) for each; every thread of the block calls.
-template <class Put>
+template <int ROWS, class Put>
 __device__ __forceinline__ void camera_tile(const CameraParams& c, int64_t n, int64_t t, const Put& put) {
-    __shared__ CamRow s_row[kCamRows];
-    __shared__ CamCol s_col[kCamCols];
-    const int64_t tile_rows = (c.h + kCamRows - 1) / kCamRows;
-    const int64_t x0 = t % tile_rows * kCamRows, y0 = t / tile_rows * kCamCols;
+    constexpr int kCols = kCamTile / ROWS;
+    __shared__ CamRow s_row[ROWS];
+    __shared__ CamCol s_col[kCols];
+    const int64_t tile_rows = (c.h + ROWS - 1) / ROWS;
+    const int64_t x0 = t % tile_rows * ROWS, y0 = t / tile_rows * kCols;
     const int i = threadIdx.x;
-    if (i < kCamRows) {
+    if (i < ROWS) {
         const double vx = ((double)(x0 + i + 1) - (double)c.h / 2.0) / c.scale;
         CamRow& q = s_row[i];
         q.a = 1.0 - vx * vx;
         q.p = -((c.p * 2.0) * vx);
         for (int k = 0; k < 3; ++k) q.r[k] = vx * (double)c.cam.right[k];
-    } else if (i >= 32 && i < 32 + kCamCols) {
-        const double vy = ((double)(y0 + i - 32 + 1) - (double)c.w / 2.0) / c.scale;
-        CamCol& q = s_col[i - 32];
+    }
+    for (int j = kCamThreads - 1 - i; j < kCols; j += kCamThreads) {  // from the other end: other warps
+        const double vy = ((double)(y0 + j + 1) - (double)c.w / 2.0) / c.scale;
+        CamCol& q = s_col[j];
         q.b = vy * vy;
         q.p = -((c.p * 2.0) * vy);
         for (int k = 0; k < 3; ++k) q.u[k] = vy * (double)c.cam.up[k];
     }
     __syncthreads();
     const float m = (float)(c.h > c.w ? c.h : c.w);
-    const int64_t x = x0 + i % kCamRows;
-    const CamRow& row = s_row[i % kCamRows];
+    const int64_t x = x0 + i % ROWS;
+    const CamRow& row = s_row[i % ROWS];
     if (x >= c.h) return;
-    for (int j = i / kCamRows; j < kCamCols; j += kCamThreads / kCamRows) {
+    for (int j = i / ROWS; j < kCols; j += kCamThreads / ROWS) {
         const int64_t g = x + c.h * (y0 + j);
         if (g >= n) return;
         const CamCol& col = s_col[j];
@@ -111,22 +117,34 @@ __device__ __forceinline__ void camera_tile(const CameraParams& c, int64_t n, in
     }
 }
 
+template <int ROWS>
 __global__ void __launch_bounds__(kCamThreads) camera_soa_kernel(CameraParams c, int64_t n, RaySoA out,
                                                                  int64_t* count) {
     if (blockIdx.x == 0 && threadIdx.x == 0) *count = n;
-    camera_tile(c, n, blockIdx.x, [&](int64_t g, const RayState& r) { store_ray(out, g, r, (uint32_t)g); });
+    camera_tile<ROWS>(c, n, blockIdx.x, [&](int64_t g, const RayState& r) { store_ray(out, g, r, (uint32_t)g); });
 }
 
+template <int ROWS>
 __global__ void __launch_bounds__(kCamThreads) camera_aos_kernel(CameraParams c, int64_t n, splat_adray_t* out) {
-    camera_tile(c, n, blockIdx.x, [&](int64_t g, const RayState& r) {
+    camera_tile<ROWS>(c, n, blockIdx.x, [&](int64_t g, const RayState& r) {
         ray_to_aos(out[g], r, kStatusActive);
         out[g].dest = g + 1;
     });
 }
 
-// Tiles of the whole h x w grid.
-static int camera_tiles(const CameraParams& c) {
-    return (int)(((c.h + kCamRows - 1) / kCamRows) * ((c.w + kCamCols - 1) / kCamCols));
+// go(rows, tiles): the tile's rows as a constant, the tiles of the whole grid.
+template <class Go>
+static void by_camera_rows(const CameraParams& c, const Go& go) {
+    auto with = [&](auto rows) {
+        const int64_t r = decltype(rows)::value, cols = kCamTile / r;
+        go(rows, (unsigned)(((c.h + r - 1) / r) * ((c.w + cols - 1) / cols)));
+    };
+    if (c.h > 16)
+        with(std::integral_constant<int, 32>{});
+    else if (c.h > 4)
+        with(std::integral_constant<int, 8>{});
+    else
+        with(std::integral_constant<int, 1>{});
 }
 
 static int grid_for_rays(int64_t n, int threads, int sm_count, int per_sm) {
@@ -138,14 +156,18 @@ static int grid_for_rays(int64_t n, int threads, int sm_count, int per_sm) {
 
 cudaError_t launch_camera_soa(const CameraParams& c, int64_t n, RaySoA out, int64_t* count, cudaStream_t s) {
     if (n <= 0) return cudaSuccess;
-    camera_soa_kernel<<<camera_tiles(c), kCamThreads, 0, s>>>(c, n, out, count);
+    by_camera_rows(c, [&](auto rows, unsigned tiles) {
+        camera_soa_kernel<decltype(rows)::value><<<tiles, kCamThreads, 0, s>>>(c, n, out, count);
+    });
     ++g_launches;
     return cudaGetLastError();
 }
 
 cudaError_t launch_camera_aos(const CameraParams& c, int64_t n, splat_adray_t* out, cudaStream_t s) {
     if (n <= 0) return cudaSuccess;
-    camera_aos_kernel<<<camera_tiles(c), kCamThreads, 0, s>>>(c, n, out);
+    by_camera_rows(c, [&](auto rows, unsigned tiles) {
+        camera_aos_kernel<decltype(rows)::value><<<tiles, kCamThreads, 0, s>>>(c, n, out);
+    });
     ++g_launches;
     return cudaGetLastError();
 }
