@@ -482,16 +482,24 @@ splat_status_t splat_server_status(const splat_server_t* server, int32_t* queued
                                    int64_t* map_bytes_in_use);
 
 /* ---------------------------------------------------------------- tuning */
-/* Launch-shape knobs (process-wide): blocks per SM of the grid-stride
- * kernels (1..256), and the splat's block-level texel aggregation (0 or 1).
- * They change only how work is spread over the GPU, never a result (float
- * maps: summation order only); the autotuner (splat_gb300/autotune.py)
- * picks them per workload. */
+/* Launch-shape knobs (process-wide): how large the grids of the grid-stride
+ * kernels may be (1..256, per SM, in the unit each line gives), and the
+ * splat's block-level texel aggregation (0 or 1).  They change only how work
+ * is spread over the GPU, never a result (float maps: summation order only);
+ * the autotuner (splat_gb300/autotune.py) picks them per workload. */
 enum {
-    SPLAT_TUNE_BRUTE_BLOCKS_PER_SM = 0, /* brute force: triangle-range splits target, in 1024 threads (default 4) */
-    SPLAT_TUNE_BVH_BLOCKS_PER_SM = 1,   /* BVH traversal grid (default 16) */
-    SPLAT_TUNE_EVOLVE_BLOCKS_PER_SM = 2, /* evolve grid (default 8) */
-    SPLAT_TUNE_SPLAT_BLOCKS_PER_SM = 3,  /* splat grid (default 8) */
+    SPLAT_TUNE_BRUTE_BLOCKS_PER_SM = 0, /* brute force: the triangle ranges are split until the launch has this many
+                                            times 1024 threads per SM, in blocks of 128 (default 4) */
+    SPLAT_TUNE_BVH_BLOCKS_PER_SM = 1,   /* BVH traversal: blocks of 128 per SM, at most as many as are resident where
+                                            rays come off a work counter; four times as many for a caller's
+                                            records, taken one ray a lane or through the two-child tree (default
+                                            16).  Launches of few rays (a group of lanes a ray) do not use it */
+    SPLAT_TUNE_EVOLVE_BLOCKS_PER_SM = 2, /* blocks of 256 per SM of ray generation, partition and the record
+                                            conversions, and of the batch engine's evolve; evolve itself takes half
+                                            of it, rounded up (default 8) */
+    SPLAT_TUNE_SPLAT_BLOCKS_PER_SM = 3,  /* splat: blocks of 160 threads per SM, launched as blocks of 128; with
+                                            SPLAT_TUNE_SPLAT_AGGREGATE and in the batch engine blocks of 256
+                                            (default 8) */
     SPLAT_TUNE_SPLAT_AGGREGATE = 4,      /* splat sums samples per texel in shared memory first (default 0) */
     SPLAT_TUNE_BVH_PACKET = 5,           /* four-wide BVH warp packets: 0 never, 1 first bounce (default), 2 every bounce,
                                             3 / 4 first bounce + per-warp choice by ray spread after (loose /

@@ -8,16 +8,17 @@
 //
 // * hit_brute_kernel: all records, behind merged boxes over 32 and 8 of them.
 //   The tiles that some ray of the block enters are staged through shared
-//   memory by TMA bulk copies (cp.async.bulk + mbarrier, 4-stage ring, no
+//   memory by TMA bulk copies (cp.async.bulk + mbarrier, two-stage ring, no
 //   multicast); each thread keeps a ray in registers and its running argmin.
 //   Record ranges split over blockIdx.y merge with a packed 64-bit atomicMin
 //   (src/atomic_argmin.jl).
 // * hit_ntris_kernel: the same rule over the reference's n_tris array, with a
-//   block's tile of records sorted and boxed on the fly.
+//   block's tile of records sorted and boxed on the fly; of few records
+//   (hit_ntris_direct_kernel) without boxes.
 // * hit_bvh_kernel: one thread per ray walks the flattened BVH2 with a short
-//   per-thread stack; boxes are padded so every triangle whose test can
-//   succeed is visited, and the same lexicographic rule makes the result
-//   identical to brute force.
+//   per-thread stack; boxes are padded, and widened by the ray's slack, so
+//   every triangle whose test can succeed is visited, and the same
+//   lexicographic rule makes the result identical to brute force.
 #include <algorithm>
 #include <cstdio>
 #include <mutex>

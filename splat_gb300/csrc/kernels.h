@@ -229,8 +229,8 @@ cudaError_t launch_refit_trees(const RefitTrees& t, const TriHit* recs, const sp
 // as two-child and four-wide nodes with leaves of at most leaf_max triangles
 constexpr int kLbvhLeaf = 4;
 size_t lbvh_scratch_bytes(int64_t n_prims);
-// (each in an array of at least n_tris - 2 nodes, at its radix-tree index),
-// with the records, boxes, order and scale launch_pack_hits would write.
+// The nodes (each in an array of at least n_tris - 2 of them, at its radix-tree
+// index), with the records, boxes, order and scale launch_pack_hits would write.
 struct LbvhOut {
     BvhNode* nodes2;
     Bvh4Node* nodes4;

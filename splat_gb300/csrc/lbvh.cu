@@ -618,8 +618,9 @@ LbvhScratch carve_lbvh(void* scratch, int64_t n) {
 size_t lbvh_scratch_bytes(int64_t np) { return np < 1 ? 256 : carve_lbvh(nullptr, np).bytes; }
 
 // 80,000 triangles: 33 launches, 250 us a rebuild -> 13 launches, 132 us;
-// 3,200: 202 -> 91; 320,000: 428 -> 282
-// (one GB300).  Before, three scan launches a sort pass, a climb of the tree
+// 3,200: 202 -> 91; 320,000: 428 -> 282; 4,000,000: 2.58 -> 2.22 ms;
+// 10,000,000, where a node near the root goes over up to 9,766 groups of 1,024
+// in turn (range_box): 7.6 -> 5.7 ms (one GB300).  Before, three scan launches a sort pass, a climb of the tree
 // for its boxes that waited on an atomic a level (52 us), and passes of their
 // own for depths, node numbering, records and boxes.
 cudaError_t launch_lbvh_build(const splat_ftri_t* ftri, int64_t n_tris, int leaf_max, void* scratch,
