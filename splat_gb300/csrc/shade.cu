@@ -40,7 +40,7 @@ namespace splat {
 // ROWS: 32, a warp's lanes being consecutive rays, for grids of more than 16
 // rows; lower ones would leave lanes idle and take 8 rows, or one.  us for
 // records of 1 x 100,000, 5 x 30,000, 9 x 20,000, 16 x 10,000 rays: without
-// tiles 41, 49, 57, 61; by 32 rows 353, 120, 87, 55; by these 37, 47, 58, 42.
+// tiles 41, 49, 57, 61; by 32 rows 353, 120, 87, 55; by these 39, 47, 55, 40.
 constexpr int kCamTile = 512;
 constexpr int kCamThreads = 256;
 
@@ -62,20 +62,24 @@ __device__ __forceinline__ void camera_tile(const CameraParams& c, int64_t n, in
     const int64_t tile_rows = (c.h + ROWS - 1) / ROWS;
     const int64_t x0 = t % tile_rows * ROWS, y0 = t / tile_rows * kCols;
     const int i = threadIdx.x;
+    auto column = [&](int j) {
+        const double vy = ((double)(y0 + j + 1) - (double)c.w / 2.0) / c.scale;
+        CamCol& q = s_col[j];
+        q.b = vy * vy;
+        q.p = -((c.p * 2.0) * vy);
+        for (int k = 0; k < 3; ++k) q.u[k] = vy * (double)c.cam.up[k];
+    };
     if (i < ROWS) {
         const double vx = ((double)(x0 + i + 1) - (double)c.h / 2.0) / c.scale;
         CamRow& q = s_row[i];
         q.a = 1.0 - vx * vx;
         q.p = -((c.p * 2.0) * vx);
         for (int k = 0; k < 3; ++k) q.r[k] = vx * (double)c.cam.right[k];
+    } else if (kCols <= kCamThreads - 32 && i >= 32 && i < 32 + kCols) {
+        column(i - 32);
     }
-    for (int j = kCamThreads - 1 - i; j < kCols; j += kCamThreads) {  // from the other end: other warps
-        const double vy = ((double)(y0 + j + 1) - (double)c.w / 2.0) / c.scale;
-        CamCol& q = s_col[j];
-        q.b = vy * vy;
-        q.p = -((c.p * 2.0) * vy);
-        for (int k = 0; k < 3; ++k) q.u[k] = vy * (double)c.cam.up[k];
-    }
+    if (kCols > kCamThreads - 32)
+        for (int j = i; j < kCols; j += kCamThreads) column(j);
     __syncthreads();
     const float m = (float)(c.h > c.w ? c.h : c.w);
     const int64_t x = x0 + i % ROWS;
