@@ -19,7 +19,7 @@
 // current best t.  The
 // BVH hitter therefore tests every triangle whose test can succeed at
 // t <= best, and with the lexicographic (t, index) rule returns exactly the
-// brute-force result.  (Compiled with -ffp-contract=off like the device
+// result of testing every triangle.  (Compiled with -ffp-contract=off like the device
 // refit, so both compute the same padded boxes.)
 #include "bvh_build.h"
 

@@ -82,3 +82,31 @@ def _lit_from_afar(res, hitter="bvh"):
 @pytest.mark.parametrize("res", [(64, 64), (160, 128)])
 def test_steps_lit_from_afar(res, hitter):
     _check(_lit_from_afar(res, hitter))
+
+
+@pytest.mark.parametrize("dist", [600.0, 2000.0])
+@pytest.mark.parametrize("turn", list(TURNS))
+@pytest.mark.parametrize("n", [1024, 4096])
+def test_brute_force(turn, dist, n):
+    """The resident brute-force hitter's boxes stand in the world's frame and
+    have their padding alone."""
+    from splat_gb300 import tracer
+
+    tris, fd, R = _scene(turn)
+    rays = _far_rays(R, dist, n, 9)
+    ref, tref = O.next_hit(rays, tris)
+    scene = tracer.Scene(tris, fd, bvh=False)
+    hit, t = tracer.next_hit(scene, tracer.BRUTE, tracer.rays_to_device(rays), with_t=True)
+    assert np.array_equal(hit.cpu().numpy(), ref)
+    assert np.array_equal(t.cpu().numpy().view(np.uint32), tref.view(np.uint32))
+    assert scene.errors() == 0
+
+
+@pytest.mark.parametrize("res", [(16, 16), (100, 90)])
+def test_brute_force_steps_lit_from_afar(res):
+    """One launch (a sponge of few facets), and separate ones."""
+    wl = _lit_from_afar(res, "brute")
+    if res[0] < 64:
+        tris, fd = S.assemble(S.menger_tris(1, 2.0, 11), S.floor_tris(-1.8, 1.5))
+        wl = wl.with_(tris=tris, first_diffuse=fd)
+    _check(wl)
