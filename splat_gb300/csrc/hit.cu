@@ -959,9 +959,11 @@ __global__ void __launch_bounds__(kBvhThreads) hit_bvh4_kernel(RaySrc src, Bvh4V
 }
 
 
-// Few rays: a warp or eight lanes a ray (bvh4_group_loop).
+// Few rays: a warp or eight lanes a ray (bvh4_group_loop).  Seven blocks share
+// an SM at 72 registers, so that kGroupRays rays of eight lanes, 1,024 blocks,
+// are one wave: 16,000 records on 81,922 triangles 45 us, 56 at six blocks.
 template <bool AOS>
-__global__ void __launch_bounds__(kBvhThreads) hit_bvh4_group_kernel(RaySrc src, Bvh4View bvh,
+__global__ void __launch_bounds__(kBvhThreads, 7) hit_bvh4_group_kernel(RaySrc src, Bvh4View bvh,
                                                                      int32_t* __restrict__ hit_idx,
                                                                      float* __restrict__ hit_t, int32_t* err) {
     __shared__ int2 s_stack[kBvhThreads / 32][kGroupStackWarp];
@@ -969,10 +971,9 @@ __global__ void __launch_bounds__(kBvhThreads) hit_bvh4_group_kernel(RaySrc src,
     if (n > kGroupRays) return;
     auto ray_of = [&](int64_t kk) { return src.perm ? (int64_t)src.perm[kk] : kk; };
     bvh4_groups(
-        n, src.fetch, s_stack[threadIdx.x >> 5], err,
-        [&](int64_t kk) { return load_hit_ray<AOS>(src, ray_of(kk)); },
-        [&](int64_t) { return bvh; },
-        [&](int64_t kk, float best, int32_t bi) {
+        (int)n, src.fetch, s_stack[threadIdx.x >> 5], err,
+        [&](int kk) { return load_hit_ray<AOS>(src, ray_of(kk)); }, bvh,
+        [&](int kk, float best, int32_t bi) {
             const int64_t k = ray_of(kk);
             hit_idx[k] = bi;
             if (hit_t) hit_t[k] = best;

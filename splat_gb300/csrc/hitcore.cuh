@@ -622,23 +622,23 @@ __device__ __forceinline__ void bvh4_group_step(const HitRay& r, const SlabRay& 
     }
 }
 
-// load(k): ray k; view(k): the BVH it is traced in; store(k, t, index).
-// Groups take rays off the work counter, or stride statically without one.
-template <int G, class Load, class View, class Store>
-__device__ __forceinline__ void bvh4_group_loop(int64_t n, unsigned long long* fetch, int2* stack, int32_t* err,
-                                                const Load& load, const View& view, const Store& store) {
+// load(k): ray k; store(k, t, index).  Groups take rays off the work counter,
+// or stride statically without one.  n is at most kGroupRays, so 32 bits hold
+// every index here.
+template <int G, class Load, class Store>
+__device__ __forceinline__ void bvh4_group_loop(int n, unsigned long long* fetch, int2* stack, int32_t* err,
+                                                const Load& load, const Bvh4View& bvh, const Store& store) {
     static_assert(G == 8 || G == 32, "group size");
     const float kInf = __int_as_float(0x7f800000);
     const int lane = threadIdx.x & 31, gl = lane & (G - 1), g0 = lane & ~(G - 1);
-    const int64_t groups = (int64_t)gridDim.x * (blockDim.x / G);
-    int64_t next = (int64_t)blockIdx.x * (blockDim.x / G) + threadIdx.x / G;
+    const int groups = (int)(gridDim.x * (blockDim.x / G));
+    int next = (int)(blockIdx.x * (blockDim.x / G) + threadIdx.x / G);
     HitRay r{};
     SlabRay sr{};
-    Bvh4View bvh{};
     float best = kInf;
     int32_t bi = 1;
     int sp = 0;
-    int64_t k = -1;  // the group's ray; -1: none
+    int k = -1;  // the group's ray; -1: none
     bool more = true;
     while (true) {
         if (sp == 0) {  // group-uniform
@@ -648,16 +648,16 @@ __device__ __forceinline__ void bvh4_group_loop(int64_t n, unsigned long long* f
         // idle groups take the next rays, one atomic per warp
         const unsigned idle = __ballot_sync(0xffffffffu, k < 0 && gl == 0);
         if (idle && more) {
-            unsigned long long base = 0;
+            int base = 0;
             if (fetch) {
-                if (lane == 0) base = atomicAdd(fetch, (unsigned long long)__popc(idle));
+                if (lane == 0) base = (int)atomicAdd(fetch, (unsigned long long)__popc(idle));
                 base = __shfl_sync(0xffffffffu, base, 0);
-                if (base + (unsigned long long)__popc(idle) >= (unsigned long long)n) more = false;
+                if (base + __popc(idle) >= n) more = false;
             }
             if (k < 0) {
-                int64_t kk;
+                int kk;
                 if (fetch) {
-                    kk = (int64_t)base + __popc(idle & ((1u << g0) - 1u));
+                    kk = base + __popc(idle & ((1u << g0) - 1u));
                 } else {
                     kk = next;
                     next += groups;
@@ -665,7 +665,6 @@ __device__ __forceinline__ void bvh4_group_loop(int64_t n, unsigned long long* f
                 if (kk < n) {
                     k = kk;
                     r = load(k);
-                    bvh = view(k);
                     sr = slab_ray(r, bvh.nodes);
                     best = kInf;
                     bi = 1;
@@ -696,13 +695,13 @@ __device__ __forceinline__ void bvh4_closest_group(const HitRay& r, bool live, c
 
 // n <= kGroupRays rays by the group size that suits their number; stack: the
 // warp's kGroupStackWarp entries.
-template <class Load, class View, class Store>
-__device__ __forceinline__ void bvh4_groups(int64_t n, unsigned long long* fetch, int2* stack, int32_t* err,
-                                            const Load& load, const View& view, const Store& store) {
+template <class Load, class Store>
+__device__ __forceinline__ void bvh4_groups(int n, unsigned long long* fetch, int2* stack, int32_t* err,
+                                            const Load& load, const Bvh4View& bvh, const Store& store) {
     if (n <= kGroupWarpRays)
-        bvh4_group_loop<32>(n, fetch, stack, err, load, view, store);
+        bvh4_group_loop<32>(n, fetch, stack, err, load, bvh, store);
     else
-        bvh4_group_loop<8>(n, fetch, stack + ((threadIdx.x & 31) >> 3) * kGroupStack<8>, err, load, view, store);
+        bvh4_group_loop<8>(n, fetch, stack + ((threadIdx.x & 31) >> 3) * kGroupStack<8>, err, load, bvh, store);
 }
 
 // Spread of a warp's rays, max over axes of (max - min) of a coordinate.
